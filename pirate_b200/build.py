@@ -14,14 +14,15 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libpirate_b200.so")
 
-SOURCES = ["plan.cpp", "avar.cpp", "simpulse.cpp", "capi.cpp", "kernels.cu", "dedisperser.cu", "noalloc.cu", "sifter.cu", "batched.cu"]
-HEADERS = ["plan.hpp", "avar.hpp", "simpulse.hpp", "yaml_lite.hpp", "kernels.cuh", "dedisperser.hpp", "regtree.cuh", "sifter.hpp", "batched.hpp"]
+SOURCES = ["plan.cpp", "avar.cpp", "simpulse.cpp", "capi.cpp", "kernels.cu", "tree_halo_f32.cu", "tree_halo_f16.cu", "tree_halo_bf16.cu", "dedisperser.cu", "noalloc.cu", "sifter.cu", "batched.cu"]
+HEADERS = ["plan.hpp", "avar.hpp", "simpulse.hpp", "yaml_lite.hpp", "kernels.cuh", "devutil.cuh", "tree_halo.cuh", "tree_halo_kernel.cuh", "dedisperser.hpp", "regtree.cuh", "sifter.hpp", "batched.hpp"]
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # -fmad=false: no fused multiply-add contraction, so the kernels perform the same fp32 roundings as
 # the reference CPU arithmetic they restate.
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-fmad=false", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
+         "--split-compile=4",
          "-Xcudafe", "--diag_suppress=177"]
 
 

@@ -188,19 +188,14 @@ void GpuDedisperser::enable_sifter(float threshold, Sifter *sf)
 }
 
 // Stage-2 launches per batch: runs of consecutive output trees with the same stage-2 kernel (same dd
-// rank and staggered-subband flag), at most kStage2MaxTrees per launch.
+// rank; all or none with subbands besides the full band), at most kStage2MaxTrees per launch.
 int GpuDedisperser::stage2_launches() const
 {
     int n = 0;
     for (long i0 = 0; i0 < plan.ntrees;) {
         long i1 = i0 + 1;
-        auto stag = [&](long i) {
-            const FrequencySubbands &fs = plan.trees[i].frequency_subbands;
-            bool x = false;
-            for (long l = 1; l <= fs.pf_rank && l < 5; l++) x = x || (fs.subband_counts[l] >= 2);
-            return x;
-        };
-        while (i1 < plan.ntrees && i1 - i0 < kStage2MaxTrees && plan.trees[i1].dd_rank == plan.trees[i0].dd_rank && stag(i1) == stag(i0)) i1++;
+        auto sub = [&](long i) { return plan.trees[i].frequency_subbands.N > 1; };   // subbands besides the full band
+        while (i1 < plan.ntrees && i1 - i0 < kStage2MaxTrees && plan.trees[i1].dd_rank == plan.trees[i0].dd_rank && sub(i1) == sub(i0)) i1++;
         n++;
         i0 = i1;
     }
@@ -348,7 +343,7 @@ void GpuDedisperser::allocate()
             st.rank = R1;
             st.nblocks = 1 << A1;
             st.nt = int(nt >> p);
-            st.state_per_block = stage1_state_floats(R1);
+            st.state_per_block = tree_block_state_floats(R1);
             add(st.state, size_t(total_beams) * st.nblocks * st.state_per_block * sizeof(float));
 
             long nrows = pow2(R1 + A1);
@@ -379,8 +374,9 @@ void GpuDedisperser::allocate()
                 for (long r = 0; r < pow2(R1); r++) {
                     long row = blk * pow2(R1) + r;
                     if (spill[row]) continue;
-                    // one sample more than the lags need: stage 2 also reads the sample before its first
-                    cap[row] = cap_r[row] = int(round_up(plan.max_row_lag[p][row] + st.nt + 1, 32));
+                    // one sample more than the lags need: stage 2 also reads the sample before its first; a
+                    // multiple of the stage-1 kernel's tile, so that no tile wraps
+                    cap[row] = cap_r[row] = int(round_up(plan.max_row_lag[p][row] + st.nt + 1, std::max(32, halo_tile(R1))));
                     off[row] = off_r[row] = tot;
                     tot += cap[row];
                 }
@@ -468,7 +464,7 @@ void GpuDedisperser::allocate()
             st.L = std::max(integer_log2(t.pf.max_width), 1);
             st.tpad = int(std::max(2 * t.pf.max_width, 4L));
             st.Dout = int(t.pf.time_downsampling);
-            st.state_per_block = stage2_state_floats(t.dd_rank);
+            st.state_per_block = tree_block_state_floats(t.dd_rank);
             add(st.state, size_t(total_beams) * st.nblocks * st.state_per_block * sizeof(float));
             int mb = 0;
             for (int l = 0; l <= fs.pf_rank; l++) {

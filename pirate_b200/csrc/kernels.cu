@@ -3,9 +3,6 @@
 //   grid_lds_kernel  tree gridding + lagged downsampling (replaces GpuTreeGriddingKernel,
 //                    src_lib/TreeGriddingKernel.cu:108-279, and GpuLaggedDownsamplingKernel,
 //                    src_lib/GpuLaggedDownsamplingKernel.cu:668-918)
-//   stage1_kernel  stage-1 tree -> delay lines   (replaces GpuDedispersionKernel outrb, src_lib/DedispersionKernel.cu:492-653)
-//   stage2_kernel  delay lines -> stage-2 tree
-//                  with subband outputs          (replaces the dd half of CoalescedDdKernel2, src_lib/CoalescedDdKernel2.cu:79-269)
 //   pf_kernel      peak finding, max/argmax      (replaces the pf half of CoalescedDdKernel2 / GpuPeakFindingKernel)
 //
 // All arithmetic is fp32 in registers with explicit round-to-nearest intrinsics (no FMA contraction),
@@ -14,9 +11,8 @@
 // out_max) is float32, float16 or bfloat16.
 
 #include "kernels.cuh"
+#include "devutil.cuh"
 
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
 #include <algorithm>
 #include <cstring>
 #include <stdexcept>
@@ -24,39 +20,6 @@
 #include <type_traits>
 
 namespace pb2 {
-
-constexpr float kRsqrt2 = 0.7071067811865476f;
-
-template<typename T> __device__ __forceinline__ float to_f(T x);
-template<> __device__ __forceinline__ float to_f<float>(float x) { return x; }
-template<> __device__ __forceinline__ float to_f<__half>(__half x) { return __half2float(x); }
-template<> __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 x) { return __bfloat162float(x); }
-
-template<typename T> __device__ __forceinline__ T from_f(float x);
-template<> __device__ __forceinline__ float from_f<float>(float x) { return x; }
-template<> __device__ __forceinline__ __half from_f<__half>(float x) { return __float2half_rn(x); }
-template<> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }
-
-__device__ __forceinline__ float bfly(float x, float y) { return __fmul_rn(kRsqrt2, __fadd_rn(x, y)); }
-
-// Tree butterflies with (NORM) or without the per-step 1/sqrt2. float32 storage normalizes at every
-// step, as the reference does, so that its outputs are bitwise the reference's. 16-bit storage keeps
-// its in-register fp32 sums unnormalized and scales once, by tree_scale(steps) = 2^(-steps/2), where a
-// value leaves the registers (a stored row or an emitted subband): one rounding instead of one per
-// step, and one multiply per stored value instead of one per butterfly.
-template<bool NORM>
-__device__ __forceinline__ float bfly_n(float x, float y) { return NORM ? bfly(x, y) : __fadd_rn(x, y); }
-
-__host__ __device__ constexpr float tree_scale(int steps)
-{
-    float s = (steps & 1) ? kRsqrt2 : 1.0f;
-    for (int i = 0; i < steps / 2; i++) s *= 0.5f;
-    return s;
-}
-
-// A value leaving the registers after n unnormalized butterflies (n is a compile-time constant at
-// every call site once the step loops are unrolled).
-__device__ __forceinline__ float tree_out(float v, int n) { return n ? __fmul_rn(v, tree_scale(n)) : v; }
 
 // Two fp32 additions (multiplications) in one sm_100 packed f32x2 instruction; each element is
 // rounded to nearest like __fadd_rn (__fmul_rn).
@@ -84,16 +47,6 @@ __device__ __forceinline__ float2 f2mul(float2 a, float2 b)
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(f2pack(a)), "l"(f2pack(b)));
     return f2unpack(d);
 }
-
-__device__ __forceinline__ int brev_bits(int x, int nbits) { return nbits ? int(__brev(unsigned(x)) >> (32 - nbits)) : 0; }
-
-static void check_launch(const char *what)
-{
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess)
-        throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
-}
-
 
 // -------------------------------------------------------------------------------------------------
 // Tree gridding fused with lagged downsampling.
@@ -778,777 +731,6 @@ __global__ void __launch_bounds__(kGridMaxThreads) grid_lds_kernel(GridLdsArgs a
 
 
 // -------------------------------------------------------------------------------------------------
-// Two-phase register trees (see regtree.cuh). Lane = time sample within a 32-sample tile.
-
-
-constexpr unsigned kFull = 0xffffffffu;
-
-// Row 'x' of the current tile lagged by L (< 32) samples, with 'p' = the same row in the previous
-// tile: the lane that holds the wanted sample offers x or p, and one shuffle delivers it.
-__device__ __forceinline__ float lagged(float x, float p, int L, int lane)
-{
-    return __shfl_sync(kFull, (lane < 32 - L) ? x : p, (lane - L) & 31);
-}
-
-template<int K> struct RT
-{
-    static constexpr int N = 1 << K;
-    static constexpr int NP = (K > 0) ? (1 << (K - 1)) : 1;
-    static constexpr int NS = (K > 0) ? K : 1;
-};
-
-// Butterfly of a lag-0 pair whose history (the previous tile's row0 at lane 31, the only lane that
-// needs it) lives in shared memory at *h instead of a register: lane 0 takes it for the lag-1
-// operand, then lane 31 stores this tile's row0. The load precedes the store in the warp's program
-// order, and the loop's __syncwarp() orders the store before the next tile's load.
-template<bool NORM>
-__device__ __forceinline__ void bfly_l0_shared(float &v0, float &v1, float *h, int lane)
-{
-    const float x = v0, y = v1, hp = *h;
-    float b = __shfl_sync(kFull, x, lane - 1);
-    b = (lane == 0) ? hp : b;
-    v0 = bfly_n<NORM>(x, y);
-    v1 = bfly_n<NORM>(b, y);
-    if (lane == 31) *h = x;
-}
-
-// Two butterflies of the same lag L at once: pair A (rows a0, a1, history pa) and pair B (rows b0, b1,
-// history pb). Row pairs (i0, i0 + 2^r) and (i0 + N/2, i0 + N/2 + 2^r) of a rank-K register tree have
-// the same lag at every step r <= K - 2, so one sm_100 packed f32x2 add does the work of two scalar
-// adds with the same rounding. The NORM multiplies stay scalar: packed multiplies by 1/sqrt2 here gave
-// outputs a few ulp from the scalar sequence on the GPU (the float32 parity tests at rank 16).
-template<bool NORM>
-__device__ __forceinline__ void bfly_x2(float &a0, float &a1, float &pa, float &b0, float &b1, float &pb, int L, int lane)
-{
-    const float xa = a0, xb = b0;
-    const float2 Y = make_float2(a1, b1);
-    const float2 A = (L == 0) ? make_float2(xa, xb) : make_float2(lagged(xa, pa, L, lane), lagged(xb, pb, L, lane));
-    const float2 Bl = make_float2(lagged(xa, pa, L + 1, lane), lagged(xb, pb, L + 1, lane));
-    float2 o0 = f2add(A, Y), o1 = f2add(Bl, Y);
-    if (NORM) {
-        o0 = make_float2(__fmul_rn(kRsqrt2, o0.x), __fmul_rn(kRsqrt2, o0.y));
-        o1 = make_float2(__fmul_rn(kRsqrt2, o1.x), __fmul_rn(kRsqrt2, o1.y));
-    }
-    a0 = o0.x; b0 = o0.y; a1 = o1.x; b1 = o1.y;
-    pa = xa; pb = xb;
-}
-
-// Step 0 with caller-supplied lag-1 operands (EXT0) for two pairs at once: (x, y) -> (x + y, e + y).
-template<bool NORM>
-__device__ __forceinline__ void bfly_ext0_x2(float &a0, float &a1, float ea, float &b0, float &b1, float eb)
-{
-    const float2 Y = make_float2(a1, b1);
-    float2 o0 = f2add(make_float2(a0, b0), Y), o1 = f2add(make_float2(ea, eb), Y);
-    if (NORM) {
-        o0 = make_float2(__fmul_rn(kRsqrt2, o0.x), __fmul_rn(kRsqrt2, o0.y));
-        o1 = make_float2(__fmul_rn(kRsqrt2, o1.x), __fmul_rn(kRsqrt2, o1.y));
-    }
-    a0 = o0.x; b0 = o0.y; a1 = o1.x; b1 = o1.y;
-}
-
-// All K steps of a register tree, in place. pv[r][q] holds pair q's row0 input of the previous tile.
-// With HS, the lag-0 pairs keep that history in shared memory (hs[slot], one float per pair, in
-// (r, q) order), which frees their registers. With EXT0, step 0 (all lags 0) takes its lag-1
-// operands from b0[q] = row 2q one sample earlier, supplied by the caller, and keeps no history;
-// with F0 the caller has already done step 0 itself (from rows it can read one sample earlier).
-// NORM: butterflies with the 1/sqrt2 (bfly_n).
-template<int K, bool HS = false, bool EXT0 = false, bool F0 = false, bool NORM = true>
-__device__ __forceinline__ void rt_steps(float (&v)[RT<K>::N], float (&pv)[RT<K>::NS][RT<K>::NP], int lane, float *hs = nullptr,
-                                         const float *b0 = nullptr)
-{
-    static_assert(!F0 || EXT0, "a caller-done step 0 keeps no history (EXT0 layout)");
-    constexpr int NP = RT<K>::NP, NH = RT<K>::N / 2;
-    int slot = 0;
-#pragma unroll
-    for (int r = 0; r < K; r++) {
-#pragma unroll
-        for (int q = 0; q < NP; q++) {
-            const int h = 1 << r;
-            const int i0 = ((q >> r) << (r + 1)) | (q & (h - 1));
-            const int L = rt_lag(r, q);
-            if (F0 && r == 0)
-                continue;
-            // Packed: pair q < NP/2 with pair q + NP/2 (rows i0 + N/2), same lag, at steps r <= K - 2.
-            const bool PK = (K >= 2) && (r <= K - 2) && !(HS && L == 0 && !(EXT0 && r == 0));
-            if (PK && q >= NP / 2)
-                continue;   // done with its partner
-            if (EXT0 && r == 0) {
-                if (PK) {
-                    bfly_ext0_x2<NORM>(v[i0], v[i0 + 1], b0[q], v[i0 + NH], v[i0 + NH + 1], b0[q + NP / 2]);
-                } else {
-                    const float x = v[i0], y = v[i0 + 1];
-                    v[i0] = bfly_n<NORM>(x, y);
-                    v[i0 + 1] = bfly_n<NORM>(b0[q], y);
-                }
-                continue;
-            }
-            if (HS && L == 0) {
-                bfly_l0_shared<NORM>(v[i0], v[i0 + h], hs + slot, lane);
-                slot++;
-                continue;
-            }
-            if (PK) {
-                bfly_x2<NORM>(v[i0], v[i0 + h], pv[r][q], v[i0 + NH], v[i0 + NH + h], pv[r][q + NP / 2], L, lane);
-                continue;
-            }
-            float x = v[i0], y = v[i0 + h];
-            float a = (L == 0) ? x : lagged(x, pv[r][q], L, lane);
-            float b = lagged(x, pv[r][q], L + 1, lane);
-            v[i0] = bfly_n<NORM>(a, y);
-            v[i0 + h] = bfly_n<NORM>(b, y);
-            pv[r][q] = x;
-        }
-    }
-}
-
-// Persistent histories: pair (r, q) needs its previous-tile row0 only in lanes >= 31 - lag.
-// With HS the lag-0 pairs' single value goes to or comes from hs[slot].
-template<int K, bool HS = false, bool EXT0 = false>
-__device__ __forceinline__ void rt_load(float (&pv)[RT<K>::NS][RT<K>::NP], const float *st, int lane, float *hs = nullptr)
-{
-    int off = 0, slot = 0;
-#pragma unroll
-    for (int r = 0; r < K; r++)
-#pragma unroll
-        for (int q = 0; q < RT<K>::NP; q++) {
-            const int L = rt_lag(r, q);
-            if (EXT0 && r == 0) {
-                // no history (its state slot stays unused)
-            } else if (HS && L == 0) {
-                if (lane == 0) hs[slot] = st[off];
-                slot++;
-            } else {
-                int i = lane - (31 - L);
-                pv[r][q] = (i >= 0) ? st[off + i] : 0.0f;
-            }
-            off += L + 1;
-        }
-    if (HS) __syncwarp();
-}
-
-template<int K, bool HS = false, bool EXT0 = false>
-__device__ __forceinline__ void rt_save(const float (&pv)[RT<K>::NS][RT<K>::NP], float *st, int lane, const float *hs = nullptr)
-{
-    if (HS) __syncwarp();
-    int off = 0, slot = 0;
-#pragma unroll
-    for (int r = 0; r < K; r++)
-#pragma unroll
-        for (int q = 0; q < RT<K>::NP; q++) {
-            const int L = rt_lag(r, q);
-            if (EXT0 && r == 0) {
-            } else if (HS && L == 0) {
-                if (lane == 0) st[off] = hs[slot];
-                slot++;
-            } else {
-                int i = lane - (31 - L);
-                if (i >= 0) st[off + i] = pv[r][q];
-            }
-            off += L + 1;
-        }
-}
-
-// Phase b of a stage-2 (subband) tree: before step r' (r' = 0..RB-1) and after it, subband rows of
-// pf level r'+1 are emitted (FrequencySubbands multiplet order), reproducing ReferenceTree::dedisperse_2d
-// (src_lib/ReferenceTree.cpp:120-300): even band pairs coincide with the in-place butterflies, odd
-// ("staggered") pairs (2k+1, 2k+2) are extra butterflies with their own histories ps[r'][u].
-// With F0 the caller has done the level-0 emission and step 0's butterflies (not its emission).
-// SA: unnormalized butterfly steps the rows have had before phase b (phase a's, or 0); NORM as in
-// rt_steps. Each emitted value is scaled by tree_scale of its unnormalized step count.
-template<int RB, bool STAG, bool HS, bool EXT0, bool F0, int SA, bool NORM, typename Emit>
-__device__ __forceinline__ void phase_b_subbands(float (&v)[1 << RB], float (&pv)[RT<RB>::NS][RT<RB>::NP],
-                                                 float (&ps)[RT<RB>::NS][RT<RB>::NP], const Stage2Args &a,
-                                                 int lane, Emit emit, float *hs, const float *b0)
-{
-    static_assert(!F0 || (EXT0 && !STAG), "a caller-done step 0: no history, no staggered pairs");
-    constexpr int NB = 1 << RB;
-    int slot = 0;   // HS: lag-0 in-place pairs keep their history in hs[slot] (see rt_steps)
-    // Band counts are the same for every tile: each level's emission is skipped as a whole when empty.
-    if (!F0 && a.sb_count[0] > 0) {
-#pragma unroll
-        for (int f = 0; f < NB; f++)
-            if (f < a.sb_count[0]) emit(a.sb_mbase[0] + f, tree_out(v[f], SA));
-    }
-
-#pragma unroll
-    for (int r = 0; r < RB; r++) {
-        const int cnt = a.sb_count[r + 1], mb = a.sb_mbase[r + 1];
-        const int h = 1 << r;
-        if (STAG && cnt >= 2) {
-#pragma unroll
-            for (int u = 0; u < (STAG ? st_count(RB, r) : 0); u++) {
-                const int k = u >> r, j = u & (h - 1);
-                if (2 * k + 1 < cnt) {
-                    const int qa = ((2 * k + 1) << r) | j, qb = ((2 * k + 2) << r) | j;
-                    const int L = rt_lag(r, j);
-                    float x = v[qa], y = v[qb];
-                    float aa = (L == 0) ? x : lagged(x, ps[r][u], L, lane);
-                    float bb = lagged(x, ps[r][u], L + 1, lane);
-                    int m = mb + (2 * k + 1) * (2 << r) + 2 * bitrev_c(j, r);
-                    emit(m, tree_out(bfly_n<NORM>(aa, y), SA + (NORM ? 0 : r + 1)));
-                    emit(m + 1, tree_out(bfly_n<NORM>(bb, y), SA + (NORM ? 0 : r + 1)));
-                    ps[r][u] = x;
-                }
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < RT<RB>::NP; q++) {
-            constexpr int NP = RT<RB>::NP, NH = NB / 2;
-            const int i0 = ((q >> r) << (r + 1)) | (q & (h - 1));
-            const int L = rt_lag(r, q);
-            // packed pairs (q, q + NP/2) as in rt_steps
-            const bool PK = (RB >= 2) && (r <= RB - 2) && !(HS && L == 0 && !(EXT0 && r == 0)) && !(F0 && r == 0);
-            if (PK && q >= NP / 2) {
-                // done with its partner
-            } else if (F0 && r == 0) {
-                // done by the caller
-            } else if (EXT0 && r == 0) {
-                if (PK) {
-                    bfly_ext0_x2<NORM>(v[i0], v[i0 + 1], b0[q], v[i0 + NH], v[i0 + NH + 1], b0[q + NP / 2]);
-                } else {
-                    const float x = v[i0], y = v[i0 + 1];
-                    v[i0] = bfly_n<NORM>(x, y);
-                    v[i0 + 1] = bfly_n<NORM>(b0[q], y);
-                }
-            } else if (PK) {
-                bfly_x2<NORM>(v[i0], v[i0 + h], pv[r][q], v[i0 + NH], v[i0 + NH + h], pv[r][q + NP / 2], L, lane);
-            } else if (HS && L == 0) {
-                bfly_l0_shared<NORM>(v[i0], v[i0 + h], hs + slot, lane);
-                slot++;
-            } else {
-                float x = v[i0], y = v[i0 + h];
-                float aa = (L == 0) ? x : lagged(x, pv[r][q], L, lane);
-                float bb = lagged(x, pv[r][q], L + 1, lane);
-                v[i0] = bfly_n<NORM>(aa, y);
-                v[i0 + h] = bfly_n<NORM>(bb, y);
-                pv[r][q] = x;
-            }
-        }
-        // Even band pairs are step r's in-place outputs.
-        if (cnt > 0) {
-#pragma unroll
-            for (int q = 0; q < RT<RB>::NP; q++) {
-                const int i0 = ((q >> r) << (r + 1)) | (q & (h - 1));
-                const int k = q >> r, j = q & (h - 1);
-                if (2 * k < cnt) {
-                    const int m = mb + (2 * k) * (2 << r) + 2 * bitrev_c(j, r);
-                    emit(m, tree_out(v[i0], SA + (NORM ? 0 : r + 1)));
-                    emit(m + 1, tree_out(v[i0 + h], SA + (NORM ? 0 : r + 1)));
-                }
-            }
-        }
-    }
-}
-
-template<int K>
-__device__ __forceinline__ void st_load(float (&ps)[RT<K>::NS][RT<K>::NP], const float *st, int lane)
-{
-    int off = 0;
-#pragma unroll
-    for (int r = 0; r < K; r++)
-#pragma unroll
-        for (int u = 0; u < RT<K>::NP; u++) {
-            if (u < st_count(K, r)) {
-                const int L = rt_lag(r, u & ((1 << r) - 1));
-                int i = lane - (31 - L);
-                ps[r][u] = (i >= 0) ? st[off + i] : 0.0f;
-                off += L + 1;
-            } else {
-                ps[r][u] = 0.0f;
-            }
-        }
-}
-
-template<int K>
-__device__ __forceinline__ void st_save(const float (&ps)[RT<K>::NS][RT<K>::NP], float *st, int lane)
-{
-    int off = 0;
-#pragma unroll
-    for (int r = 0; r < K; r++)
-#pragma unroll
-        for (int u = 0; u < RT<K>::NP; u++) {
-            if (u < st_count(K, r)) {
-                const int L = rt_lag(r, u & ((1 << r) - 1));
-                int i = lane - (31 - L);
-                if (i >= 0) st[off + i] = ps[r][u];
-                off += L + 1;
-            }
-        }
-}
-
-template<typename Ts>
-struct PfEmit
-{
-    Ts *row0;   // multiplet 0 of this warp's coarse dm, at the current tile's slot + lane
-    int cap;    // delay line capacity (multiplet stride)
-    __device__ __forceinline__ void operator()(int m, float v) const
-    {
-        row0[m * cap] = from_f<Ts>(v);
-    }
-};
-
-// Shared-memory delay line between the phases: row rr = f * 2^RA + d (f < 2^RB) starts at float
-// off(rr) and has capacity cap(rr) = ring_cap(f, d), a multiple of 32. Phase a writes tile k at
-// wpos, phase b reads tile k-1 at rpos - P(f, d); positions are multiples of 32, so a write never
-// wraps and a read wraps at most once. Per row the tables hold
-//   wb[f * 2^RA + d] = off + wpos                 (phase a: write index of lane 0)
-//   rt[d * 2^RB + f] = {off + rpos - P, off | cap << 16}   (phase b: read index of lane 0, wrap bounds)
-// so that each warp's rows are consecutive (128-bit table loads).
-template<int RA, int RB>
-__device__ __forceinline__ int ring_lag(int f, int d) { return ((1 << RB) - 1 - f) * brev_bits(d, RA); }
-
-__device__ __forceinline__ int wrap_add(int p, int cap) { return (p >= cap) ? (p - cap) : ((p < 0) ? (p + cap) : p); }
-
-// Entry i of a warp's consecutive table row (16-byte aligned base; four ints or two int2 per 128-bit
-// shared load, the fields selected at compile time in the unrolled loops that call these).
-// N = entries per row: 128-bit loads need N a multiple of 4 (int) or 2 (int2), which keeps every
-// row base 16-byte aligned; smaller rows use plain loads.
-template<int N>
-__device__ __forceinline__ int tab_int(const int *base, int i)
-{
-    if constexpr (N % 4 != 0) {
-        return base[i];
-    } else {
-        const int4 t = ((const int4 *) base)[i >> 2];
-        return ((i & 3) == 0) ? t.x : ((i & 3) == 1) ? t.y : ((i & 3) == 2) ? t.z : t.w;
-    }
-}
-template<int N>
-__device__ __forceinline__ int2 tab_int2(const int2 *base, int i)
-{
-    if constexpr (N % 2 != 0) {
-        return base[i];
-    } else {
-        const int4 t = ((const int4 *) base)[i >> 1];
-        return (i & 1) ? make_int2(t.z, t.w) : make_int2(t.x, t.y);
-    }
-}
-
-// Fills wb[] and rt[] for stream time s0 (a multiple of 32). Uses ioff[NR] as scratch; ends with
-// __syncthreads().
-template<int RA, int RB>
-__device__ void ring_init(int *wb, int2 *rt, int *ioff, long s0)
-{
-    constexpr int NR = 1 << (RA + RB);
-    const int rr = threadIdx.x;
-    const int f = rr >> RA, d = rr & ((1 << RA) - 1);
-    if (rr < NR)
-        ioff[rr] = ring_cap(RA, RB, f, d);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int o = 0;
-        for (int i = 0; i < NR; i++) {
-            const int c = ioff[i];
-            ioff[i] = o;
-            o += c;
-        }
-    }
-    __syncthreads();
-    if (rr < NR) {
-        const int off = ioff[rr], cap = ring_cap(RA, RB, f, d), P = ring_lag<RA, RB>(f, d);
-        const int pos = int(s0 % cap);
-        wb[rr] = off + pos;
-        rt[d * (1 << RB) + f] = make_int2(off + pos - P, off | (cap << 16));
-    }
-    __syncthreads();
-}
-
-template<int BYTES>
-__device__ __forceinline__ void cp_async_bytes(void *smem, const void *gmem)
-{
-    unsigned s = (unsigned) __cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" :: "r"(s), "l"(gmem), "n"(BYTES) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-// Staging of one tile of a phase-a warp's NA input rows: 32-bit words copied with cp.async.
-// float: 32 words per row; 16-bit types: 17 words (34 samples) starting at an even sample.
-// Staging of one tile of input rows with 16-byte cp.async copies of EPC samples. Stage-1 rows are
-// read aligned (32 samples); a stage-2 row starts at an arbitrary sample p and is copied as the
-// EPC-aligned run of 32 + EPC samples from p & ~(EPC-1) (SPR samples per staged row).
-template<typename Ts> struct Stage
-{
-    static constexpr int EPC = 16 / sizeof(Ts);
-    static constexpr int SPR = 32 + EPC;
-};
-
-// Shared-memory layout of a two-phase tree kernel (byte offsets; host and device agree).
-template<typename Ts, int RA, int RB>
-struct TreeSmem
-{
-    static constexpr int NR = 1 << (RA + RB);
-    static_assert(NR >= 2 && ring_floats(RA, RB) < 65536, "delay-line tables pack offset and capacity in 16 bits");
-    static constexpr size_t in_tab = 0;                       // int4[NR]
-    static constexpr size_t out_base = in_tab + 16 * NR;      // int[NR]
-    static constexpr size_t out_off = out_base + 4 * NR;      // int[NR]
-    static constexpr size_t rt = out_off + 4 * NR;            // int2[NR]
-    static constexpr size_t wb = rt + 8 * NR;                 // int[NR]
-    static constexpr size_t in_cap = wb + 4 * NR;             // int[NR]
-    static constexpr size_t hist = in_cap + 4 * NR;           // float[warps][16]: lag-0 histories
-    static constexpr size_t staging = (hist + 4 * 16 * ((1 << RA) + (1 << RB)) + 15) & ~size_t(15);
-    static constexpr size_t ring = (staging + 2 * (1 << RB) * (1 << RA) * Stage<Ts>::SPR * sizeof(Ts) + 15) & ~size_t(15);
-    static constexpr size_t total = ring + sizeof(float) * ring_floats(RA, RB);
-};
-
-// Lag-0 histories in shared memory (HS in rt_steps) for the rank-7 and rank-8 trees, whose register
-// budgets (64 and 80 per thread in 1024- and 768-thread blocks) are the tightest.
-__host__ __device__ constexpr bool tree_hs(int RA, int RB, int STAGE) { return RA + RB >= 7; }
-
-template<int STAGE>
-struct TreeArgsOf;
-template<> struct TreeArgsOf<1> { using type = Stage1Args; };
-template<> struct TreeArgsOf<2> { using type = Stage2Args; };
-
-// Launch parameter: one stage-1 tree, or a grid of stage-2 trees (Stage2Multi).
-template<int STAGE>
-struct TreeParamOf;
-template<> struct TreeParamOf<1> { using type = Stage1Args; };
-template<> struct TreeParamOf<2> { using type = Stage2Multi; };
-
-template<int STAGE, typename PT>
-__device__ __forceinline__ const typename TreeArgsOf<STAGE>::type &tree_args(const PT &P, int ti)
-{
-    if constexpr (STAGE == 1) return P;
-    else return P.t[ti];
-}
-
-// Two-phase tree kernel. Warps [0, NB) run phase a on tile k while warps [NB, NB+NA) run phase b on
-// tile k-1; one block barrier per tile.
-//   STAGE 1: input = level-p tree rows (aligned), output = per-row stage-1 delay lines.
-//   STAGE 2: input = stage-1 delay lines read at lag rb_lag (misaligned), output = subband rows.
-template<typename Ts, int RA, int RB, int STAGE, bool STAG, bool HS = tree_hs(RA, RB, STAGE)>
-__global__ void __launch_bounds__(32 * ((1 << RA) + (1 << RB)), 1) tree_kernel(const __grid_constant__ typename TreeParamOf<STAGE>::type P)
-{
-    // Stage 2: this block's tree ti and its block index blk among that tree's nblk blocks.
-    int ti = 0, blk = blockIdx.x, nblk = gridDim.x;
-    if constexpr (STAGE == 2) {
-        while (ti + 1 < P.n && blk >= P.blk0[ti + 1]) ti++;
-        nblk = P.blk0[ti + 1] - P.blk0[ti];
-        blk -= P.blk0[ti];
-    }
-    const auto &a = tree_args<STAGE>(P, ti);
-    constexpr int NA = 1 << RA, NB = 1 << RB, NR = 1 << (RA + RB);
-    constexpr int RING = ring_floats(RA, RB);
-    // Staging row stride: stage-1 rows are 32 aligned samples; stage-2 rows take one more chunk.
-    constexpr int SPRK = (STAGE == 1) ? 32 : Stage<Ts>::SPR;
-    using Lay = TreeSmem<Ts, RA, RB>;
-    extern __shared__ __align__(16) unsigned char sm_raw[];
-
-    // stage 2, per input row: {read position, capacity, offset low and high words} of its delay line
-    int4 *in_tab = (int4 *) (sm_raw + Lay::in_tab);
-    // stage 1, per output row (f, d) at [d * NB + f]: index of lane 0 and start of its delay line,
-    // relative to the block's first line
-    int *out_base = (int *) (sm_raw + Lay::out_base);
-    int *out_off = (int *) (sm_raw + Lay::out_off);
-    int2 *rt = (int2 *) (sm_raw + Lay::rt);
-    int *wb = (int *) (sm_raw + Lay::wb);
-    int *in_cap = (int *) (sm_raw + Lay::in_cap);         // stage 1: output delay line capacities
-    Ts *staging = (Ts *) (sm_raw + Lay::staging);
-    float *ring = (float *) (sm_raw + Lay::ring);
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float *hs = (float *) (sm_raw + Lay::hist) + warp * 16;   // this warp's lag-0 histories (HS)
-    // Step 0 (all lags 0) without shuffles or histories. Stage 1, phase b: the lag-1 operands are read
-    // from the shared delay line. Stage 2: each phase does step 0 while it loads its rows, phase a
-    // reading each row from one sample earlier in the staging buffer (rows are staged from p - 1)
-    // and phase b from the delay line, so no extra values stay live.
-    constexpr bool E0 = (STAGE == 1);
-    constexpr bool FA = (STAGE == 2) && (RA >= 1);
-    constexpr bool FB = (STAGE == 2) && !STAG && (RB >= 1);
-    constexpr bool EB = E0 || FB;
-    // bfly_n per phase: float32 storage normalizes every step. 16-bit storage skips the 1/sqrt2 in both
-    // phases of both stages (measured 4%, 2% and, with the packed adds, 2% faster in stage 2's phase b)
-    // and scales by tree_scale(SU) where values leave the registers.
-    constexpr bool NORM_A = (sizeof(Ts) == 4);
-    constexpr bool NORM_B = (sizeof(Ts) == 4);
-    constexpr int SA = NORM_A ? 0 : RA;                 // unnormalized steps before phase b
-    constexpr int SU = SA + (NORM_B ? 0 : RB);          // ... and after it
-    const int b = blockIdx.y, bt = a.beam0 + b;
-    float *st = a.state + ((long) bt * nblk + blk) * a.state_per_block;
-
-    // The shared delay line comes back from HBM with 16-byte cp.async copies (RING is a multiple of 32
-    // floats, and each block's state starts on a 16-byte boundary), overlapping the table setup below;
-    // each thread waits for its copies before the block barrier that ends the setup.
-    const bool st16 = ((reinterpret_cast<uintptr_t>(st) & 15) == 0);
-    if (st16) {
-        for (int i = threadIdx.x; i < RING / 4; i += blockDim.x)
-            cp_async_bytes<16>(ring + 4 * i, st + 4 * i);
-        cp_async_commit();
-    } else {
-        for (int i = threadIdx.x; i < RING; i += blockDim.x)
-            ring[i] = st[i];
-    }
-    const long s0 = a.chunk_ctr ? *a.chunk_ctr * (long) a.nt : a.s0;
-    ring_init<RA, RB>(wb, rt, in_cap, s0);
-
-    const Ts *in;
-    int pos1 = 0;   // stage 1: read position of every input row (rows are read aligned)
-    if constexpr (STAGE == 1) {
-        in = (const Ts *) a.in + (long) (a.in_beam0 + b) * a.in_beam_stride + (long) blk * NR * a.in_row_stride;
-        pos1 = int(((a.chunk_ctr && a.in_mask != -1) ? s0 : a.in_s0) & a.in_mask);
-        const long off0 = a.ring_off[(long) blk * NR];   // the host checks that a block's lines span < 2^31
-        for (int r = threadIdx.x; r < NR; r += blockDim.x) {
-            const int cap = a.ring_cap[(long) blk * NR + r];   // capacity of output delay line r (a multiple of 32)
-            const int off = int(a.ring_off[(long) blk * NR + r] - off0);
-            const int j = (r & (NA - 1)) * NB + (r >> RA);      // row (f, d) = r at [d * NB + f]
-            in_cap[j] = cap;
-            out_off[j] = off;
-            out_base[j] = off + int(s0 % cap);
-        }
-    } else {
-        in = (const Ts *) a.ring + (long) bt * a.ring_beam_stride;
-        const long dm1 = brev_bits(blk, a.amb_rank) + (a.uflag ? (1L << a.amb_rank) : 0L);
-        for (int r = threadIdx.x; r < NR; r += blockDim.x) {
-            long row = ((long) r << a.amb_rank) + blk;
-            long lag = (long) (NR - 1 - r) * dm1;
-            long cap = a.ring_cap[row];
-            long p = (s0 - lag) % cap;
-            const long off = a.ring_off[row];
-            in_tab[r] = make_int4(int(p < 0 ? p + cap : p), int(cap), int(off & 0xffffffffL), int(off >> 32));
-        }
-    }
-
-    const bool is_a = warp < NB;
-    const int g = is_a ? warp : (warp - NB);   // phase-a group (f) or phase-b group (d)
-    const int ntiles = a.nt / 32;
-    cp_async_wait0();
-    __syncthreads();
-    // Register splits between the warp roles (whole warpgroups: phase a is warps 0-15). Each block is
-    // launched with the kernel's allocation, and the split adds up to exactly that, so the increasing
-    // role's request is always satisfied once the other role has decreased, which each of its warps
-    // does here before any barrier:
-    //   4+4 (1024 threads, 64 registers): 72 x 512 (phase a) + 56 x 512 (phase b) = 64 x 1024, or
-    //        56 x 512 + 72 x 512 for stage 2 with staggered subband pairs (phase b's extra histories);
-    //   3+4 (768 threads, 80 registers): 72 x 512 (phase a) + 96 x 256 (phase b) = 80 x 768.
-    if constexpr (RA == 4 && RB == 4 && !(STAGE == 2 && STAG)) {
-        if (is_a) asm volatile("setmaxnreg.inc.sync.aligned.u32 72;");
-        else asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-    }
-    if constexpr (RA == 4 && RB == 4 && STAGE == 2 && STAG) {
-        if (is_a) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-        else asm volatile("setmaxnreg.inc.sync.aligned.u32 72;");
-    }
-    if constexpr (RA == 3 && RB == 4) {
-        if (is_a) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-        else asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
-    }
-
-    // The two warp roles run separate loops (so each holds only its own histories in registers);
-    // they meet once per tile at named barrier 1.
-    if (is_a) {
-        float pva[RT<RA>::NS][RT<RA>::NP];
-        float *sta = st + RING + g * rt_state(RA);
-        // Phase a keeps its lag-0 histories in registers where the split gives it the room (measured
-        // faster); with staggered subbands it has 56 registers and keeps them in shared memory.
-        constexpr bool HSA = HS && !(RB == 4 && (RA == 4 || RA == 3) && !(STAGE == 2 && STAG));
-        rt_load<RA, HSA, FA>(pva, sta, lane, hs);
-
-        // Issues the cp.async copies of this warp's NA rows for one tile into staging buffer 'buf',
-        // then advances the rows' read positions by 32 samples.
-        Ts *my_stage = staging + g * NA * SPRK;
-        auto issue = [&](int buf) {
-            Ts *dst = my_stage + buf * NB * NA * SPRK;
-            if constexpr (STAGE == 1) {
-                // Aligned rows at a common position: 16-byte copies, CH per row.
-                constexpr int EPC = 16 / sizeof(Ts), CH = 32 / EPC;
-                for (int c = lane; c < NA * CH; c += 32) {
-                    const int i = c / CH, k = c % CH;
-                    cp_async_bytes<16>(dst + i * SPRK + k * EPC, in + (long) (g * NA + i) * a.in_row_stride + pos1 + k * EPC);
-                }
-                pos1 = int((pos1 + 32) & a.in_mask);
-            } else {
-                // Rows at their own positions: CPR consecutive 16-byte chunks from p & ~(EPC-1), consecutive
-                // lanes on consecutive chunks of a row. Capacities are multiples of 32 samples, so a chunk
-                // never straddles the end of a delay line and wraps at most once.
-                // With FA the run starts at p - 1 (32 + 1 samples fit in the same CPR chunks).
-                constexpr int EPC = Stage<Ts>::EPC, CPR = 32 / EPC + 1;
-                for (int c = lane; c < NA * CPR; c += 32) {
-                    const int i = c / CPR, k = c - i * CPR, r = g * NA + i;
-                    const int4 t = in_tab[r];
-                    const int cap = t.y;
-                    const int p0 = FA ? ((t.x == 0) ? (cap - 1) : (t.x - 1)) : t.x;
-                    int q = (p0 & ~(EPC - 1)) + k * EPC;
-                    q = (q >= cap) ? (q - cap) : q;
-                    cp_async_bytes<16>(dst + i * SPRK + k * EPC, in + ((long) t.w << 32 | (unsigned) t.z) + q);
-                }
-                __syncwarp();
-                if (lane < NA) {
-                    const int rr = g * NA + lane;
-                    in_tab[rr].x = wrap_add(in_tab[rr].x + 32, in_tab[rr].y);
-                }
-            }
-            __syncwarp();
-        };
-
-        // Stage 2: bits [OB i, OB i + OB) = offset in its staged run of the first staged sample of row i,
-        // (p - FA) & (EPC-1) (constant: positions advance by 32 and capacities are multiples of 32).
-        constexpr int OB = (sizeof(Ts) == 4) ? 2 : 3;
-        unsigned long long offs = 0;
-        if (STAGE == 2) {
-#pragma unroll
-            for (int i = 0; i < NA; i++)
-                offs |= (unsigned long long) ((in_tab[g * NA + i].x - (FA ? 1 : 0)) & (Stage<Ts>::EPC - 1)) << (OB * i);
-        }
-        issue(0);
-        cp_async_commit();
-
-        for (int it = 0; it <= ntiles; it++) {
-            if (it < ntiles) {
-                if (it + 1 < ntiles) issue((it + 1) & 1);
-                cp_async_commit();
-                cp_async_wait1();
-                __syncwarp();
-                const Ts *sb = my_stage + (it & 1) * NB * NA * SPRK;
-                float v[NA];
-                if constexpr (FA) {
-                    // Step 0 while loading: pair (2q, 2q + 1), lag-1 operand = row 2q one sample earlier.
-#pragma unroll
-                    for (int q = 0; q < NA / 2; q++) {
-                        const Ts *r0 = sb + 2 * q * SPRK + lane + int((offs >> (OB * 2 * q)) & ((1u << OB) - 1));
-                        const Ts *r1 = sb + (2 * q + 1) * SPRK + lane + int((offs >> (OB * (2 * q + 1))) & ((1u << OB) - 1));
-                        const float xm = to_f(r0[0]), x = to_f(r0[1]), y = to_f(r1[1]);
-                        v[2 * q] = bfly_n<NORM_A>(x, y);
-                        v[2 * q + 1] = bfly_n<NORM_A>(xm, y);
-                    }
-                    rt_steps<RA, HSA, true, true, NORM_A>(v, pva, lane, hs);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < NA; i++)
-                        v[i] = to_f(sb[i * SPRK + lane + int((offs >> (OB * i)) & ((1u << OB) - 1))]);
-                    rt_steps<RA, HSA, false, false, NORM_A>(v, pva, lane, hs);
-                }
-#pragma unroll
-                for (int i = 0; i < NA; i++)
-                    ring[tab_int<NA>(wb + g * NA, i) + lane] = v[i];
-                __syncwarp();
-                if (lane < NA) {
-                    const int rr = g * NA + lane;
-                    const int y = rt[lane * NB + g].y;   // phase b updates only rt[].x
-                    const int lo = y & 0xffff, cap = y >> 16;
-                    const int w = wb[rr] + 32;
-                    wb[rr] = (w == lo + cap) ? lo : w;
-                }
-            }
-            asm volatile("bar.sync 1, %0;" :: "r"(blockDim.x) : "memory");
-        }
-        cp_async_wait0();
-        rt_save<RA, HSA, FA>(pva, sta, lane, hs);
-    } else {
-        float pvb[RT<RB>::NS][RT<RB>::NP], psb[RT<RB>::NS][RT<RB>::NP];
-        float *stb = st + RING + NB * rt_state(RA) + g * (rt_state(RB) + (STAGE == 2 ? st_state(RB) : 0));
-        // Phase b keeps its lag-0 histories in shared memory (56 registers, or 72 with staggered pairs,
-        // whose own histories take the room), except in the 3+4 trees, where it has 96.
-        constexpr bool HSB = HS && !(RA == 3 && RB == 4);
-        rt_load<RB, HSB, EB>(pvb, stb, lane, hs);
-        if (STAG) st_load<RB>(psb, stb + rt_state(RB), lane);
-
-        PfEmit<Ts> emit;
-        Ts *pf_rows = nullptr;   // stage 2: multiplet 0 of this warp's coarse dm
-        int pf_slot = 0;         // stage 2: delay-line slot of this lane's sample in the current tile
-        if constexpr (STAGE == 2) {
-            const int pf_dm = brev_bits(g, RA);
-            const long rowbase = ((long) bt * a.ndm_out + ((long) brev_bits(blk, a.amb_rank) << RA) + pf_dm) * a.M;
-            pf_rows = (Ts *) a.pf + rowbase * a.pf_cap;
-            pf_slot = int((s0 + lane) & (a.pf_cap - 1));
-            emit.cap = int(a.pf_cap);
-        }
-
-        for (int it = 0; it <= ntiles; it++) {
-            if (it >= 1) {
-                // Phase-b rows, and (E0) for step 0 (lag 0) each even row one sample earlier: the delay
-                // line holds it (capacity >= P + 65), so no shuffle and no history are needed.
-                float v[NB], b0[RT<RB>::NP];
-                if constexpr (FB || (STAGE == 1 && RB >= 1)) {
-                    // Step 0 while loading (pair (f, f + 1), lag-1 operand = row f one sample earlier,
-                    // from the delay line), and in stage 2 the level-0 emission.
-                    int cnt0 = 0, mb0 = 0;
-                    if constexpr (STAGE == 2) {
-                        emit.row0 = pf_rows + pf_slot;
-                        pf_slot = (pf_slot + 32) & int(a.pf_cap - 1);
-                        cnt0 = a.sb_count[0];
-                        mb0 = a.sb_mbase[0];
-                    }
-#pragma unroll
-                    for (int f = 0; f < NB; f += 2) {
-                        const int2 t0 = tab_int2<NB>(rt + g * NB, f), t1 = tab_int2<NB>(rt + g * NB, f + 1);
-                        const int lo0 = t0.y & 0xffff, cap0 = t0.y >> 16, lo1 = t1.y & 0xffff, cap1 = t1.y >> 16;
-                        int q0 = t0.x + lane, q1 = t1.x + lane;
-                        q0 = (q0 < lo0) ? (q0 + cap0) : q0;
-                        q1 = (q1 < lo1) ? (q1 + cap1) : q1;
-                        const int qm = (q0 == lo0) ? (q0 + cap0 - 1) : (q0 - 1);
-                        const float x = ring[q0], y = ring[q1], xm = ring[qm];
-                        if (STAGE == 2 && cnt0 > 0) {
-                            if (f < cnt0) emit(mb0 + f, tree_out(x, SA));
-                            if (f + 1 < cnt0) emit(mb0 + f + 1, tree_out(y, SA));
-                        }
-                        v[f] = bfly_n<NORM_B>(x, y);
-                        v[f + 1] = bfly_n<NORM_B>(xm, y);
-                    }
-                } else {
-#pragma unroll
-                    for (int f = 0; f < NB; f++) {
-                        const int2 t = tab_int2<NB>(rt + g * NB, f);
-                        const int lo = t.y & 0xffff, cap = t.y >> 16;
-                        int q = t.x + lane;
-                        q = (q < lo) ? (q + cap) : q;
-                        v[f] = ring[q];
-                        if (E0 && (f & 1) == 0 && RB > 0) {
-                            const int qm = (q == lo) ? (q + cap - 1) : (q - 1);
-                            b0[f >> 1] = ring[qm];
-                        }
-                    }
-                }
-                __syncwarp();
-                if (lane < NB) {
-                    const int rr = g * NB + lane;   // row (f = lane, d = g)
-                    const int2 t = rt[rr];
-                    const int lo = t.y & 0xffff, cap = t.y >> 16;
-                    const int x = t.x + 32;
-                    rt[rr].x = (x >= lo + cap - ring_lag<RA, RB>(lane, g)) ? (x - cap) : x;
-                }
-                if constexpr (STAGE == 1) {
-                    if constexpr (RB >= 1)
-                        rt_steps<RB, HSB, true, true, NORM_B>(v, pvb, lane, hs);
-                    else
-                        rt_steps<RB, HSB, E0, false, NORM_B>(v, pvb, lane, hs, b0);
-                    Ts *out = (Ts *) a.ring + (long) bt * a.ring_beam_stride + a.ring_off[(long) blk * NR];
-#pragma unroll
-                    for (int f = 0; f < NB; f++)
-                        out[tab_int<NB>(out_base + g * NB, f) + lane] = from_f<Ts>(tree_out(v[f], SU));
-                    __syncwarp();
-                    if (lane < NB) {
-                        const int i = g * NB + lane;
-                        const int ob = out_base[i] + 32;
-                        out_base[i] = (ob == out_off[i] + in_cap[i]) ? out_off[i] : ob;
-                    }
-                } else if constexpr (FB) {
-                    phase_b_subbands<RB, STAG, HSB, true, true, SA, NORM_B>(v, pvb, psb, a, lane, emit, hs, b0);
-                } else {
-                    emit.row0 = pf_rows + pf_slot;
-                    pf_slot = (pf_slot + 32) & int(a.pf_cap - 1);
-                    phase_b_subbands<RB, STAG, HSB, E0, false, SA, NORM_B>(v, pvb, psb, a, lane, emit, hs, b0);
-                }
-            }
-            asm volatile("bar.sync 1, %0;" :: "r"(blockDim.x) : "memory");
-        }
-        rt_save<RB, HSB, EB>(pvb, stb, lane, hs);
-        if (STAG) st_save<RB>(psb, stb + rt_state(RB), lane);
-    }
-    __syncthreads();
-
-    if (st16) {
-        for (int i = threadIdx.x; i < RING / 4; i += blockDim.x)
-            reinterpret_cast<float4 *>(st)[i] = reinterpret_cast<const float4 *>(ring)[i];
-    } else {
-        for (int i = threadIdx.x; i < RING; i += blockDim.x)
-            st[i] = ring[i];
-    }
-}
-
-
-// -------------------------------------------------------------------------------------------------
 // Peak finding. One warp per (beam, coarse dm, 32 consecutive output times). For each multiplet m
 // the warp stages the input window in shared memory and builds the boxcar levels with the reference's
 // recursion  B_{l+1}[u] = B_l[r u] + B_l[r u + s]  (so every boxcar sum has the reference's rounding);
@@ -2216,63 +1398,24 @@ void launch_grid_lds(const GridLdsArgs &a, int dtype, cudaStream_t s)
     else launch_grid_lds_d<__nv_bfloat16>(a, s);
 }
 
-template<typename Ts, int RA, int RB>
-static size_t tree_smem()
-{
-    return TreeSmem<Ts, RA, RB>::total;
-}
-
-template<typename K>
-static void set_smem(K kernel, size_t bytes)
-{
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes);
-    if (e != cudaSuccess) throw std::runtime_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
-}
-
-template<typename Ts, int R, int STAGE, bool STAG, typename A>
-static void launch_tree_r(const A &a, int nblocks, int B, cudaStream_t s)
-{
-    constexpr int RA = split_ra(R), RB = split_rb(R);
-    size_t sm = tree_smem<Ts, RA, RB>();
-    set_smem(tree_kernel<Ts, RA, RB, STAGE, STAG>, sm);
-    tree_kernel<Ts, RA, RB, STAGE, STAG><<<dim3(nblocks, B), tree_threads(R), sm, s>>>(a);
-    check_launch(STAGE == 1 ? "stage1 tree_kernel" : "stage2 tree_kernel");
-}
-
-template<typename Ts, int STAGE, bool STAG, typename A>
-static void launch_tree_t(const A &a, int rank, int nblocks, int B, cudaStream_t s)
-{
-    switch (rank) {
-    case 1: launch_tree_r<Ts, 1, STAGE, STAG>(a, nblocks, B, s); break;
-    case 2: launch_tree_r<Ts, 2, STAGE, STAG>(a, nblocks, B, s); break;
-    case 3: launch_tree_r<Ts, 3, STAGE, STAG>(a, nblocks, B, s); break;
-    case 4: launch_tree_r<Ts, 4, STAGE, STAG>(a, nblocks, B, s); break;
-    case 5: launch_tree_r<Ts, 5, STAGE, STAG>(a, nblocks, B, s); break;
-    case 6: launch_tree_r<Ts, 6, STAGE, STAG>(a, nblocks, B, s); break;
-    case 7: launch_tree_r<Ts, 7, STAGE, STAG>(a, nblocks, B, s); break;
-    case 8: launch_tree_r<Ts, 8, STAGE, STAG>(a, nblocks, B, s); break;
-    default: throw std::runtime_error("tree_kernel: unsupported dd rank " + std::to_string(rank));
-    }
-}
-
 void launch_stage1(const Stage1Args &a, int dtype, int nblocks, int B, cudaStream_t s)
 {
     if (a.in_lag0 != 0 || a.in_lag1 != 0) throw std::runtime_error("launch_stage1: input rows must be aligned (no read lag)");
-    if (dtype == 0) launch_tree_t<float, 1, false>(a, a.rank, nblocks, B, s);
-    else if (dtype == 1) launch_tree_t<__half, 1, false>(a, a.rank, nblocks, B, s);
-    else launch_tree_t<__nv_bfloat16, 1, false>(a, a.rank, nblocks, B, s);
+    if (dtype == 0) launch_stage1_halo_f32(a, nblocks, B, s);
+    else if (dtype == 1) launch_stage1_halo_f16(a, nblocks, B, s);
+    else launch_stage1_halo_bf16(a, nblocks, B, s);
 }
 
-static bool stage2_staggered(const Stage2Args &a)
+static bool stage2_full_band(const Stage2Args &a)
 {
-    bool stag = false;
-    for (int l = 1; l < 5; l++) stag = stag || (a.sb_count[l] >= 2);
-    return stag;
+    for (int l = 0; l < split_rb(a.rank) && l < 5; l++)
+        if (a.sb_count[l] != 0) return false;
+    return true;
 }
 
 bool stage2_same_kernel(const Stage2Args &x, const Stage2Args &y)
 {
-    return x.rank == y.rank && stage2_staggered(x) == stage2_staggered(y);
+    return x.rank == y.rank && stage2_full_band(x) == stage2_full_band(y);
 }
 
 void launch_stage2_multi(const Stage2Args *a, const int *nblocks, int n, int dtype, int B, cudaStream_t s)
@@ -2291,15 +1434,10 @@ void launch_stage2_multi(const Stage2Args *a, const int *nblocks, int n, int dty
     }
     if (tot > (1L << 30)) throw std::runtime_error("launch_stage2_multi: grid too large");
     m.blk0[n] = int(tot);
-    if (stage2_staggered(a[0])) {
-        if (dtype == 0) launch_tree_t<float, 2, true>(m, a[0].rank, int(tot), B, s);
-        else if (dtype == 1) launch_tree_t<__half, 2, true>(m, a[0].rank, int(tot), B, s);
-        else launch_tree_t<__nv_bfloat16, 2, true>(m, a[0].rank, int(tot), B, s);
-    } else {
-        if (dtype == 0) launch_tree_t<float, 2, false>(m, a[0].rank, int(tot), B, s);
-        else if (dtype == 1) launch_tree_t<__half, 2, false>(m, a[0].rank, int(tot), B, s);
-        else launch_tree_t<__nv_bfloat16, 2, false>(m, a[0].rank, int(tot), B, s);
-    }
+    const bool sub = !stage2_full_band(a[0]);
+    if (dtype == 0) launch_stage2_halo_f32(m, sub, int(tot), B, s);
+    else if (dtype == 1) launch_stage2_halo_f16(m, sub, int(tot), B, s);
+    else launch_stage2_halo_bf16(m, sub, int(tot), B, s);
 }
 
 void launch_stage2(const Stage2Args &a, int dtype, int nblocks, int B, cudaStream_t s)

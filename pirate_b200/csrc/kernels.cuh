@@ -14,13 +14,6 @@ namespace pb2 {
 __host__ __device__ constexpr int split_rb(int R) { return (R + 1) / 2; }
 __host__ __device__ constexpr int split_ra(int R) { return R - (R + 1) / 2; }
 
-// Threads per block of a two-phase tree kernel of rank R: one warp per phase-a group (2^RB of
-// them) followed by one warp per phase-b group (2^RA).
-__host__ __device__ constexpr int tree_threads(int R)
-{
-    return 32 * ((1 << split_ra(R)) + (1 << split_rb(R)));
-}
-
 // Stage 1 (one primary tree): input rows -> two-phase tree -> per-row output delay lines.
 struct Stage1Args
 {
@@ -124,11 +117,8 @@ struct GridLdsArgs
     int block_target;       // threads per block to aim for (0: 128); blocks hold whole rows of windows
 };
 
-// Floats of persistent state per block of the stage kernels (host and device agree by construction).
-// Per-block state, rounded up to a multiple of 4 floats so that every block's state starts on a
-// 16-byte boundary (the kernels move its delay-line part with 16-byte copies).
-inline long stage1_state_floats(int R) { return (tree_state_floats(split_ra(R), split_rb(R), false) + 3) & ~3L; }
-inline long stage2_state_floats(int R) { return (tree_state_floats(split_ra(R), split_rb(R), true) + 3) & ~3L; }
+// Floats of persistent state per block of the tree kernels.
+inline long tree_block_state_floats(int R) { return halo_state_floats(split_ra(R), split_rb(R)); }
 
 // Per-beam peak of a batch's outputs, as pirate's toy grouper reduces them (pirate_frb/run_toy_grouper.py:
 // 79-116): over every tree, the maximum of out_max[tree][b] and its first (dm, time) position; a tree
@@ -192,9 +182,9 @@ void launch_dequantize(void *out, int out_dtype, const void *data, const void *s
 void launch_stage1(const Stage1Args &a, int dtype, int nblocks, int B, cudaStream_t s);
 void launch_stage2(const Stage2Args &a, int dtype, int nblocks, int B, cudaStream_t s);
 
-// Stage 2 of several output trees that use the same kernel (same dd rank and staggered-subband flag)
-// as one grid: blocks [blk0[i], blk0[i+1]) are tree i's. One grid has one partial last wave instead of
-// one per tree (the downsampled trees' grids are 3.5 waves).
+// Stage 2 of several output trees that use the same kernel (same dd rank; all or none with subbands besides
+// the full band) as one grid: blocks [blk0[i], blk0[i+1]) are tree i's. One grid has one partial last wave
+// instead of one per tree (the downsampled trees' grids are 3.5 waves).
 constexpr int kStage2MaxTrees = 8;
 struct Stage2Multi
 {
@@ -204,6 +194,13 @@ struct Stage2Multi
 };
 bool stage2_same_kernel(const Stage2Args &x, const Stage2Args &y);
 void launch_stage2_multi(const Stage2Args *a, const int *nblocks, int n, int dtype, int B, cudaStream_t s);
+// One translation unit per storage type (tree_halo_*.cu).
+void launch_stage1_halo_f32(const Stage1Args &a, int nblocks, int B, cudaStream_t s);
+void launch_stage1_halo_f16(const Stage1Args &a, int nblocks, int B, cudaStream_t s);
+void launch_stage1_halo_bf16(const Stage1Args &a, int nblocks, int B, cudaStream_t s);
+void launch_stage2_halo_f32(const Stage2Multi &m, bool sub, int nblocks, int B, cudaStream_t s);
+void launch_stage2_halo_f16(const Stage2Multi &m, bool sub, int nblocks, int B, cudaStream_t s);
+void launch_stage2_halo_bf16(const Stage2Multi &m, bool sub, int nblocks, int B, cudaStream_t s);
 void launch_pf(const PfArgs &a, int dtype, int B, cudaStream_t s);
 
 struct DedispersionPlan;

@@ -142,7 +142,7 @@ void dedisperse_chunk_noalloc(const DedispersionPlan &plan, const void *in, cons
         }
         st.ring_off_t = tab.put(off.data(), nrows * sizeof(long));
         st.ring_cap_t = tab.put(cap.data(), nrows * sizeof(int));
-        st.state_pb = stage1_state_floats(R1);
+        st.state_pb = tree_block_state_floats(R1);
         st.lds_cap = (p > 0) ? na_pow2_ceil(st.nt + (1L << R1) - 1) : 0;
     }
     for (long i = 0; i < plan.ntrees; i++) {
@@ -158,7 +158,7 @@ void dedisperse_chunk_noalloc(const DedispersionPlan &plan, const void *in, cons
         st.L = std::max(integer_log2(t.pf.max_width), 1);
         st.tpad = int(std::max(2 * t.pf.max_width, 4L));
         st.Dout = int(t.pf.time_downsampling);
-        st.state_pb = stage2_state_floats(t.dd_rank);
+        st.state_pb = tree_block_state_floats(t.dd_rank);
         int mb = 0;
         for (int l = 0; l < 5; l++) { st.cnt[l] = 0; st.mb[l] = 0; }
         for (int l = 0; l <= fs.pf_rank; l++) { st.cnt[l] = int(fs.subband_counts[l]); st.mb[l] = mb; mb += int(fs.subband_counts[l]) << l; }

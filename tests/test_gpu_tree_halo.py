@@ -1,0 +1,61 @@
+"""The tree kernels at the edges of their tiles: float32 outputs must equal the fp32 oracle's bit for bit.
+
+Tiles are the largest power of two up to 64-256 samples (by tree rank) that divides the chunk, segments 512-2048
+samples; blocks read their rows at every alignment. The cases take chunks of one short tile, of an odd number of
+tiles, longer than a segment, every dd rank from 1 to 8, full-band and (staggered) subband outputs."""
+
+import numpy as np
+import pytest
+
+import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+# (rank, nt, subbands, primary trees as (early triggers, max width), chunks)
+CASES = [
+    (3, 32, [1], [(0, 4)], 9),                         # dd ranks 1 + 2, one 32-sample tile
+    (4, 96, [0, 1], [(1, 4)], 7),                      # dd ranks 2 + 1, 2; three 32-sample tiles
+    (5, 352, [1, 1], [(2, 8)], 4),                     # dd ranks 2 + 1..3
+    (6, 4160, [0, 0, 1], [(1, 8), (0, 4)], 2),         # 64-sample tiles of long-tile trees, segments of 2048
+    (9, 2560, [0, 0, 0, 1], [(0, 16), (0, 8)], 2),     # dd ranks 4, 5: a segment and a quarter
+    (10, 448, [4, 7, 3, 1], [(1, 8)], 4),              # every subband level, staggered pairs
+    (12, 192, [0, 3, 0, 1], [(1, 16), (0, 8)], 4),     # dd ranks 5, 6, odd tiles
+    (14, 640, [0, 0, 0, 0, 1], [(0, 8), (0, 4)], 2),   # dd rank 7: segments of 2048 (float32), odd tiles
+    (16, 1088, [0, 1, 0, 0, 1], [(0, 8)], 2),          # dd rank 8: a float32 segment (1024) and one tile
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "r%d_t%d" % (c[0], c[1]))
+def test_tree_tiles_bitwise(pb2lib, case):
+    rank, nt, sb, pts, nchunks = case
+    prim = []
+    for ip, (net, w) in enumerate(pts):
+        prim.append(dict(num_early_triggers=net, max_width=w, dm_downsampling=0, time_downsampling=0,
+                         wt_dm_downsampling=2 ** ((rank - (1 if ip else 0) - net + 1) // 2), wt_time_downsampling=16))
+    cfg = H.toy_config(rank=rank, nfreq=max(8, 2 ** rank // 3), nt=nt, subbands=sb, beams_per_gpu=1, beams_per_batch=1,
+                       primary_trees=prim)
+    xs = H.make_inputs(cfg, nchunks, seed=rank + nt)
+    orc, _ = H.run_oracle(cfg, xs[:0], [])
+    ws = H.make_weights(orc, seed=rank)
+    _, ores = H.run_oracle(cfg, xs, ws, 1, 32)
+    _, _, gres = H.run_gpu(pb2lib, cfg, xs, ws)
+    for seq in range(nchunks):
+        for i in range(orc.ntrees):
+            assert np.array_equal(gres[seq][0][i], ores[seq][0][i]), "out_max, chunk %d tree %d" % (seq, i)
+            assert np.array_equal(gres[seq][1][i], ores[seq][1][i]), "out_argmax, chunk %d tree %d" % (seq, i)
+
+
+@pytest.mark.parametrize("dtype,tol", [("float16", 1e-2), ("bfloat16", 6e-2)])
+def test_tree_tiles_16bit(pb2lib, dtype, tol):
+    """16-bit rows start at any sample of a 16-byte chunk; against the FP64 oracle, in sigma (bare weights)."""
+    cfg = H.toy_config(rank=13, nfreq=3000, nt=192, dtype=dtype, subbands=[0, 3, 0, 1], beams_per_gpu=1, beams_per_batch=1,
+                       primary_trees=[dict(num_early_triggers=1, max_width=8, dm_downsampling=0, time_downsampling=0,
+                                           wt_dm_downsampling=64, wt_time_downsampling=16)])
+    xs = H.make_inputs(cfg, 4, seed=3)
+    orc, _ = H.run_oracle(cfg, xs[:0], [])
+    ws = H.make_weights(orc, seed=3, kind="bare")
+    _, ores = H.run_oracle(cfg, xs, ws, 1, 64)
+    _, _, gres = H.run_gpu(pb2lib, cfg, xs, ws)
+    for seq in range(4):
+        for i in range(orc.ntrees):
+            assert np.abs(gres[seq][0][i] - ores[seq][0][i]).max() <= tol
