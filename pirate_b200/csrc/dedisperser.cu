@@ -124,8 +124,8 @@ void GpuDedisperser::stop(std::exception_ptr e)
 
 int GpuDedisperser::kernels_per_batch() const
 {
-    // candidate stage: beam peaks, patches, then the MLP (3 GEMMs) and the score mask, or the mask alone
-    const int cand = sift ? (3 + (sifter ? 4 : 1)) : 0;
+    // candidate stage: beam peaks (2), patches, then the MLP (2 kernels) and the score mask, or the mask alone
+    const int cand = sift ? (3 + (sifter ? 3 : 1)) : 0;
     int spill = 0;
     for (const Stage1 &st : s1) spill += st.nspill ? 2 : 0;
     return 1 + int(plan.num_primary_trees) + spill + stage2_launches() + int(plan.ntrees) + cand;

@@ -2,6 +2,7 @@
 
 #include "sifter.hpp"
 
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -111,197 +112,440 @@ void launch_mask_scores(const float *logits, const int *valid, float *scores, in
 }
 
 // ---------------------------------------------------------------------------------------------
-// GEMM on the tensor cores: C = A B^T (+ bias), bf16 operands, FP32 accumulation.
-// A element (m, k) at A[m*sam + k*sak], B element (n, k) at B[n*sbn + k*sbk], either stored as float,
-// fp16 or bf16 (rounded to bf16 while staged in shared memory). 64x64 block tiles, K steps of 32,
-// four warps of 32x32, each issuing mma.sync.m16n8k16 (row.col, bf16 -> f32).
-// Outputs: C (f32, optional) = acc; Cb (bf16, optional) = relu ? max(acc, 0) : acc.
+// The MLP on the tensor cores: bf16 operands, FP32 accumulation (mma.sync m16n8k16). At 1 MFLOP per candidate and
+// at most 1024 candidates the work is bound by latency, so the kernels are few and wide. (One GEMM kernel per product,
+// its K loop of 32-wide steps unpipelined, took about 24 launches and 620 us per training step of 512, and 0.4 ms for
+// the 8 candidates of a chunk; these take 3 launches and about 120 us with the host's part, and 38 us with the patches.)
+//   layer1_kernel  Z1 = X W1^T + b1, H1 = bf16(relu(Z1)): 32 x 32 tiles, K in chunks of 64 through a cp.async
+//                  pipeline, split over the blocks of a cluster where a small batch has few tiles
+//   head_kernel    16 candidates per block: layers 2 and 3, and in training everything between the logits and
+//                  the two large weight gradients (loss, g2, g1, partial bias and W3 gradients)
+//   wgrad_kernel   dW1 = g1^T X and dW2 = g2^T H1 in 64 x 64 tiles, with the Adam step in the epilogue
 
-struct GemmArgs
-{
-    int M, N, K;
-    const void *A; long sam, sak;
-    const void *B; long sbn, sbk;
-    const float *bias;
-    int relu;
-    float *C; long ldc;
-    uint16_t *Cb; long ldcb;
-};
+constexpr int kIn = kMlpIn, kH1 = kMlpH1, kH2 = kMlpH2;
+constexpr int kKc = 64, kKPitch = kKc + 8;    // K chunk; padded row of a staged tile (ldmatrix without bank conflicts)
+constexpr int kStages = 3;
+constexpr int kHeadRows = 16;
 
-constexpr int kGBM = 64, kGBN = 64, kGBK = 32, kGPad = 8;
-
-__device__ __forceinline__ void mma_bf16(float *c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
 {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const void *p)
+{
+    const unsigned a = (unsigned) __cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], const void *p)
+{
+    const unsigned a = (unsigned) __cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+// 16-byte asynchronous copy, zeros when !ok (the source is then not read).
+__device__ __forceinline__ void cp16(void *dst, const void *src, bool ok)
+{
+    const unsigned d = (unsigned) __cvta_generic_to_shared(dst);
+    const int n = ok ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" :: "r"(d), "l"(src), "r"(n) : "memory");
+}
+// Eight 16-bit values of an input row that need not start on a 16-byte boundary.
+__device__ __forceinline__ void copy8(uint16_t *dst, const uint16_t *src, bool ok, bool aligned)
+{
+    if (aligned) {
+        cp16(dst, src, ok);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; i++) dst[i] = ok ? src[i] : 0;
+    }
+}
+__device__ __forceinline__ uint32_t half2_to_bf162(uint32_t h)
+{
+    const float2 f = __half22float2(*(const __half2 *) &h);
+    const __nv_bfloat162 b = __floats2bfloat162_rn(f.x, f.y);
+    return *(const uint32_t *) &b;
+}
+__device__ __forceinline__ float relu(float x) { return (x < 0.0f) ? 0.0f : x; }   // NaN passes
+__device__ __forceinline__ float bf_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+__device__ __forceinline__ uint16_t bf_bits(float x)
+{
+    const __nv_bfloat16 h = __float2bfloat16_rn(x);
+    return *(const uint16_t *) &h;
+}
+__device__ __forceinline__ float bf_float(uint16_t b) { return __uint_as_float(uint32_t(b) << 16); }
+
+template<int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" :: "n"(N) : "memory"); }
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+
+struct Layer1Args
+{
+    const uint16_t *x, *w;   // fp16 (n, kIn), bf16 (kH1, kIn)
+    const float *bias;
+    int n, aligned;
+    float *z;
+    uint16_t *h;
+};
+
+// Grid (kH1 / 32, row blocks, S) in clusters of the S blocks of one tile; block z sums the K chunks
+// [27 z / S, 27 (z + 1) / S), and the blocks of a cluster then add each other's tiles in rank order.
+__global__ void __launch_bounds__(128) layer1_kernel(Layer1Args g)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    __shared__ __align__(16) uint16_t As[kStages][32][kKPitch], Bs[kStages][32][kKPitch];
+    __shared__ float red[32][33];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n0 = blockIdx.x * 32, m0 = blockIdx.y * 32, z = blockIdx.z, S = gridDim.z;
+    constexpr int NC = kIn / kKc;
+    const int c0 = NC * z / S, c1 = NC * (z + 1) / S;
+    auto load = [&](int c) {
+        if (c < c1) {
+            const int st = c % kStages;
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const int i = tid + 128 * j, r = i >> 3, k = (i & 7) * 8;
+                const bool ok = m0 + r < g.n;
+                copy8(&As[st][r][k], g.x + (long) (ok ? m0 + r : 0) * kIn + c * kKc + k, ok, g.aligned);
+                cp16(&Bs[st][r][k], g.w + (long) (n0 + r) * kIn + c * kKc + k, true);
+            }
+        }
+        cp_commit();
+    };
+    for (int c = c0; c < c0 + kStages - 1; c++) load(c);
+    const int wm = (warp >> 1) * 16, wn = (warp & 1) * 16;
+    float acc[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+    for (int c = c0; c < c1; c++) {
+        cp_wait<kStages - 2>();
+        __syncthreads();
+        load(c + kStages - 1);   // into the buffer that was read before this barrier
+        const int st = c % kStages;
+#pragma unroll
+        for (int ks = 0; ks < kKc; ks += 16) {
+            uint32_t a[4], b[4];
+            ldsm4(a, &As[st][wm + (lane & 15)][ks + (lane >> 4) * 8]);
+            ldsm4(b, &Bs[st][wn + (lane >> 4) * 8 + (lane & 7)][ks + ((lane >> 3) & 1) * 8]);
+#pragma unroll
+            for (int i = 0; i < 4; i++) a[i] = half2_to_bf162(a[i]);
+            mma_bf16(acc[0], a, b[0], b[1]);
+            mma_bf16(acc[1], a, b[2], b[3]);
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < 2; t++)
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            red[wm + (lane >> 2) + (q >> 1) * 8][wn + t * 8 + (lane & 3) * 2 + (q & 1)] = acc[t][q];
+    if (S > 1) cl.sync();
+    else __syncthreads();
+    for (int i = 1024 * z / S + tid; i < 1024 * (z + 1) / S; i += 128) {
+        const int r = i >> 5, c = i & 31;
+        if (m0 + r >= g.n) continue;
+        float v = 0.0f;
+        if (S > 1) {
+            for (int k = 0; k < S; k++) v += cl.map_shared_rank(&red[0][0], k)[r * 33 + c];
+        } else {
+            v = red[r][c];
+        }
+        v += g.bias[n0 + c];
+        const long o = (long) (m0 + r) * kH1 + n0 + c;
+        g.z[o] = v;
+        g.h[o] = bf_bits(relu(v));
+    }
+    if (S > 1) cl.sync();   // no block ends while another reads its tile
 }
 
-template<typename TA, typename TB>
-__global__ void __launch_bounds__(128) gemm_kernel(GemmArgs g)
-{
-    __shared__ __align__(16) __nv_bfloat16 As[kGBM][kGBK + kGPad];
-    __shared__ __align__(16) __nv_bfloat16 Bs[kGBN][kGBK + kGPad];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = warp >> 1, wn = warp & 1;
-    const int gid = lane >> 2, tig = lane & 3;
-    const int m0 = blockIdx.y * kGBM, n0 = blockIdx.x * kGBN;
-    const TA *A = (const TA *) g.A;
-    const TB *B = (const TB *) g.B;
+// Partial sums of a head block: db1 [0, 256), db2 [256, 384), dW3 [384, 512), db3 512, loss 513.
+constexpr int kPart = kH1 + 2 * kH2 + 2;
 
+struct HeadArgs
+{
+    const uint16_t *h1, *w2, *w3;   // bf16
+    const float *z1, *b2, *b3;
+    int n;
+    float *logits;           // inference
+    const float *labels;     // training (null: inference)
+    uint16_t *g1, *g2;       // bf16 (n, kH1), (n, kH2)
+    float *part;             // (blocks, kPart)
+};
+
+struct HeadSmem
+{
+    uint16_t h1[kHeadRows][kH1 + 8];
+    uint16_t w2[kH2][kH1 + 8];
+    float z2[kHeadRows][kH2 + 4];
+    uint16_t g2[kHeadRows][kH2 + 8];
+    float w3[kH2];
+    float g[kHeadRows], ls[kHeadRows];
+};
+
+__global__ void __launch_bounds__(256) head_kernel(HeadArgs g)
+{
+    extern __shared__ __align__(16) unsigned char head_sm[];
+    HeadSmem &s = *(HeadSmem *) head_sm;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int r0 = blockIdx.x * kHeadRows;
+    for (int i = tid; i < kHeadRows * (kH1 / 8); i += 256) {
+        const int r = i / (kH1 / 8), k = i % (kH1 / 8) * 8;
+        const bool ok = r0 + r < g.n;
+        cp16(&s.h1[r][k], g.h1 + (long) (ok ? r0 + r : 0) * kH1 + k, ok);
+    }
+    for (int i = tid; i < kH2 * (kH1 / 8); i += 256) {
+        const int r = i / (kH1 / 8), k = i % (kH1 / 8) * 8;
+        cp16(&s.w2[r][k], g.w2 + (long) r * kH1 + k, true);
+    }
+    cp_commit();
+    if (tid < kH2) s.w3[tid] = bf_float(g.w3[tid]);
+    cp_wait<0>();
+    __syncthreads();
+    {
+        // Z2 = H1 W2^T + b2: warp w takes 16 columns
+        float acc[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+        const int c0 = warp * 16;
+#pragma unroll
+        for (int ks = 0; ks < kH1; ks += 16) {
+            uint32_t a[4], b[4];
+            ldsm4(a, &s.h1[lane & 15][ks + (lane >> 4) * 8]);
+            ldsm4(b, &s.w2[c0 + (lane >> 4) * 8 + (lane & 7)][ks + ((lane >> 3) & 1) * 8]);
+            mma_bf16(acc[0], a, b[0], b[1]);
+            mma_bf16(acc[1], a, b[2], b[3]);
+        }
+#pragma unroll
+        for (int t = 0; t < 2; t++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int c = c0 + t * 8 + (lane & 3) * 2 + (q & 1);
+                s.z2[(lane >> 2) + (q >> 1) * 8][c] = acc[t][q] + g.b2[c];
+            }
+    }
+    __syncthreads();
+    // logit = H2 W3^T + b3: 16 threads per row
+    const int row = tid >> 4, part = tid & 15;
+    float v = 0.0f;
+#pragma unroll
+    for (int j = 0; j < kH2 / 16; j++) {
+        const int c = part + 16 * j;
+        v += bf_round(relu(s.z2[row][c])) * s.w3[c];
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    const float logit = v + g.b3[0];
+    const bool live = r0 + row < g.n;
+    if (!g.labels) {
+        if (part == 0 && live) g.logits[r0 + row] = logit;
+        return;
+    }
+    // Mean binary cross-entropy; g = (sigmoid(z) - y) / n
+    if (part == 0) {
+        float gi = 0.0f, l = 0.0f;
+        if (live) {
+            const float y = g.labels[r0 + row];
+            const float sig = 1.0f / (1.0f + expf(-logit));
+            gi = (sig - y) / (float) g.n;
+            l = fmaxf(logit, 0.0f) - logit * y + log1pf(expf(-fabsf(logit)));
+        }
+        s.g[row] = gi;
+        s.ls[row] = l;
+    }
+    __syncthreads();
+    float *pt = g.part + (long) blockIdx.x * kPart;
+    if (tid < kH2) {
+        // g2 = (g W3) masked by Z2 > 0; column sums over the block's rows for db2 and dW3
+        float db2 = 0.0f, dw3 = 0.0f;
+#pragma unroll
+        for (int r = 0; r < kHeadRows; r++) {
+            const float gr = bf_round(s.g[r]), z = s.z2[r][tid];
+            const float g2 = (z > 0.0f) ? gr * s.w3[tid] : 0.0f;
+            db2 += g2;
+            dw3 += gr * bf_round(relu(z));
+            const uint16_t h = bf_bits(g2);
+            s.g2[r][tid] = h;
+            if (r0 + r < g.n) g.g2[(long) (r0 + r) * kH2 + tid] = h;
+        }
+        pt[kH1 + tid] = db2;
+        pt[kH1 + kH2 + tid] = dw3;
+    } else if (tid == kH2) {
+        float db3 = 0.0f, l = 0.0f;
+        for (int r = 0; r < kHeadRows; r++) { db3 += s.g[r]; l += s.ls[r]; }
+        pt[kH1 + 2 * kH2] = db3;
+        pt[kH1 + 2 * kH2 + 1] = l;
+    }
+    __syncthreads();
+    // g1 = (g2 W2) masked by Z1 > 0: warp w takes 32 columns
+    float acc[4][4];
+#pragma unroll
+    for (int t = 0; t < 4; t++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) acc[t][q] = 0.0f;
+    const int c0 = warp * 32;
+#pragma unroll
+    for (int ks = 0; ks < kH2; ks += 16) {
+        uint32_t a[4], b[4];
+        ldsm4(a, &s.g2[lane & 15][ks + (lane >> 4) * 8]);
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+            ldsm4t(b, &s.w2[ks + (lane & 15)][c0 + p * 16 + (lane >> 4) * 8]);
+            mma_bf16(acc[2 * p], a, b[0], b[1]);
+            mma_bf16(acc[2 * p + 1], a, b[2], b[3]);
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+        float cs[2] = {0.0f, 0.0f};
+        const int c = c0 + t * 8 + (lane & 3) * 2;
+#pragma unroll
+        for (int hh = 0; hh < 2; hh++) {
+            const int r = r0 + (lane >> 2) + hh * 8;
+            if (r < g.n) {
+                const float2 z = *(const float2 *) (g.z1 + (long) r * kH1 + c);
+                const float v0 = (z.x > 0.0f) ? acc[t][2 * hh] : 0.0f, v1 = (z.y > 0.0f) ? acc[t][2 * hh + 1] : 0.0f;
+                cs[0] += v0;
+                cs[1] += v1;
+                *(uint32_t *) (g.g1 + (long) r * kH1 + c) = uint32_t(bf_bits(v0)) | (uint32_t(bf_bits(v1)) << 16);
+            }
+        }
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) {
+            cs[0] += __shfl_xor_sync(0xffffffffu, cs[0], o);
+            cs[1] += __shfl_xor_sync(0xffffffffu, cs[1], o);
+        }
+        if (lane < 4) { pt[c] = cs[0]; pt[c + 1] = cs[1]; }
+    }
+}
+
+struct WgradArgs
+{
+    const uint16_t *g1, *g2, *h1, *x;   // bf16 (n, kH1), (n, kH2), (n, kH1); fp16 (n, kIn)
+    const float *part;
+    int n, nparts, aligned;
+    float *loss;
+    float *grad;                        // null: Adam step instead
+    float *w, *m, *v;                   // fp32 parameters and moments
+    uint16_t *wb;                       // bf16 copies of W1, W2, W3
+    float lr, c1, c2;
+};
+
+static constexpr long kW1n = long(kMlpH1) * kMlpIn, kW2n = long(kMlpH2) * kMlpH1;
+static constexpr long oW1 = 0, oB1 = oW1 + kW1n, oW2 = oB1 + kMlpH1, oB2 = oW2 + kW2n, oW3 = oB2 + kMlpH2, oB3 = oW3 + kMlpH2;
+static constexpr long kNparams = oB3 + 1;
+static constexpr long bW1 = 0, bW2 = kW1n, bW3 = kW1n + kW2n, kNbf16 = kW1n + kW2n + kMlpH2;
+
+// The gradient gi of parameter i (bf16 copy at wb[ib], ib < 0: none): stored, or one Adam step (0.9, 0.999, 1e-8).
+__device__ __forceinline__ void take_grad(const WgradArgs &g, long i, long ib, float gi)
+{
+    if (g.grad) {
+        g.grad[i] = gi;
+        return;
+    }
+    const float mi = 0.9f * g.m[i] + 0.1f * gi;
+    const float vi = 0.999f * g.v[i] + 0.001f * gi * gi;
+    g.m[i] = mi;
+    g.v[i] = vi;
+    const float wi = g.w[i] - g.lr * (mi / g.c1) / (sqrtf(vi / g.c2) + 1.0e-8f);
+    g.w[i] = wi;
+    if (ib >= 0) g.wb[ib] = bf_bits(wi);
+}
+
+constexpr int kWgK = 32;                             // candidates per pipeline step
+constexpr int kWgTiles1 = (kMlpH1 / 64) * (kMlpIn / 64), kWgTiles2 = (kMlpH2 / 64) * (kMlpH1 / 64);
+
+// C(m, c) = sum_k A[k][m] B[k][c] over the n candidates, 64 x 64 tiles, four warps of 32 x 32; operands are read
+// as they lie (candidates in rows) and transposed by ldmatrix. The last block reduces the head blocks' partials.
+__global__ void __launch_bounds__(128) wgrad_kernel(WgradArgs g)
+{
+    __shared__ __align__(16) uint16_t As[kStages][kWgK][kKPitch], Bs[kStages][kWgK][kKPitch];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int blk = blockIdx.x;
+    if (blk == kWgTiles1 + kWgTiles2) {
+        for (int i = tid; i < kPart; i += 128) {
+            float v = 0.0f;
+            for (int p = 0; p < g.nparts; p++) v += g.part[(long) p * kPart + i];
+            if (i < kH1) take_grad(g, oB1 + i, -1, v);
+            else if (i < kH1 + kH2) take_grad(g, oB2 + i - kH1, -1, v);
+            else if (i < kH1 + 2 * kH2) take_grad(g, oW3 + i - kH1 - kH2, bW3 + i - kH1 - kH2, v);
+            else if (i == kH1 + 2 * kH2) take_grad(g, oB3, -1, v);
+            else g.loss[0] = v / (float) g.n;
+        }
+        return;
+    }
+    const bool first = blk < kWgTiles1;
+    if (!first) blk -= kWgTiles1;
+    const int lda = first ? kH1 : kH2, ldb = first ? kIn : kH1;
+    const int tn = ldb / 64, m0 = blk / tn * 64, c0 = blk % tn * 64;
+    const uint16_t *A = first ? g.g1 : g.g2, *B = first ? g.x : g.h1;
+    const bool al = first ? g.aligned : true;
+    const int nk = (g.n + kWgK - 1) / kWgK;
+    auto load = [&](int c) {
+        if (c < nk) {
+            const int st = c % kStages;
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const int i = tid + 128 * j, r = i >> 3, k = (i & 7) * 8;
+                const bool ok = c * kWgK + r < g.n;
+                const long rr = ok ? c * kWgK + r : 0;
+                cp16(&As[st][r][k], A + rr * lda + m0 + k, ok);
+                copy8(&Bs[st][r][k], B + rr * ldb + c0 + k, ok, al);
+            }
+        }
+        cp_commit();
+    };
+    for (int c = 0; c < kStages - 1; c++) load(c);
+    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
     float acc[2][4][4];
 #pragma unroll
     for (int i = 0; i < 2; i++)
 #pragma unroll
-        for (int jj = 0; jj < 4; jj++)
+        for (int t = 0; t < 4; t++)
 #pragma unroll
-            for (int q = 0; q < 4; q++) acc[i][jj][q] = 0.0f;
-
-    for (int k0 = 0; k0 < g.K; k0 += kGBK) {
-#pragma unroll 4
-        for (int e = tid; e < kGBM * kGBK; e += 128) {
-            const int r = e / kGBK, c = e % kGBK;
-            const int m = m0 + r, k = k0 + c;
-            const float va = (m < g.M && k < g.K) ? sf_to_f(A[(long) m * g.sam + (long) k * g.sak]) : 0.0f;
-            As[r][c] = __float2bfloat16_rn(va);
-            const int n = n0 + r;
-            const float vb = (n < g.N && k < g.K) ? sf_to_f(B[(long) n * g.sbn + (long) k * g.sbk]) : 0.0f;
-            Bs[r][c] = __float2bfloat16_rn(vb);
-        }
+            for (int q = 0; q < 4; q++) acc[i][t][q] = 0.0f;
+    for (int c = 0; c < nk; c++) {
+        cp_wait<kStages - 2>();
         __syncthreads();
+        load(c + kStages - 1);
+        const int st = c % kStages;
 #pragma unroll
-        for (int ks = 0; ks < kGBK; ks += 16) {
-            uint32_t af[2][4], bfr[4][2];
+        for (int ks = 0; ks < kWgK; ks += 16) {
+            uint32_t a[2][4], b[2][4];
 #pragma unroll
-            for (int mt = 0; mt < 2; mt++) {
-                const int r0 = wm * 32 + mt * 16 + gid;
-                const int c0 = ks + tig * 2;
-                af[mt][0] = *(const uint32_t *) &As[r0][c0];
-                af[mt][1] = *(const uint32_t *) &As[r0 + 8][c0];
-                af[mt][2] = *(const uint32_t *) &As[r0][c0 + 8];
-                af[mt][3] = *(const uint32_t *) &As[r0 + 8][c0 + 8];
-            }
+            for (int i = 0; i < 2; i++) {
+                ldsm4t(a[i], &As[st][ks + (lane >> 4) * 8 + (lane & 7)][wm + i * 16 + ((lane >> 3) & 1) * 8]);
+                ldsm4t(b[i], &Bs[st][ks + (lane & 15)][wn + i * 16 + (lane >> 4) * 8]);
+                if (first) {
 #pragma unroll
-            for (int nt = 0; nt < 4; nt++) {
-                const int n = wn * 32 + nt * 8 + gid;
-                const int k = ks + tig * 2;
-                bfr[nt][0] = *(const uint32_t *) &Bs[n][k];
-                bfr[nt][1] = *(const uint32_t *) &Bs[n][k + 8];
-            }
-#pragma unroll
-            for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-                for (int nt = 0; nt < 4; nt++)
-                    mma_bf16(acc[mt][nt], af[mt][0], af[mt][1], af[mt][2], af[mt][3], bfr[nt][0], bfr[nt][1]);
-        }
-        __syncthreads();
-    }
-
-#pragma unroll
-    for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-        for (int nt = 0; nt < 4; nt++)
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int m = m0 + wm * 32 + mt * 16 + gid + ((q >> 1) ? 8 : 0);
-                const int n = n0 + wn * 32 + nt * 8 + tig * 2 + (q & 1);
-                if (m < g.M && n < g.N) {
-                    float v = acc[mt][nt][q] + (g.bias ? g.bias[n] : 0.0f);
-                    if (g.C) g.C[(long) m * g.ldc + n] = v;
-                    if (g.Cb) {
-                        const float r = (g.relu && v < 0.0f) ? 0.0f : v;
-                        __nv_bfloat16 h = __float2bfloat16_rn(r);
-                        g.Cb[(long) m * g.ldcb + n] = *(const uint16_t *) &h;
-                    }
+                    for (int q = 0; q < 4; q++) b[i][q] = half2_to_bf162(b[i][q]);
                 }
             }
-}
-
-enum { kF32 = 0, kF16 = 1, kBF16 = 2 };
-
-static void gemm(const GemmArgs &g, int ta, int tb, cudaStream_t s)
-{
-    if (g.M <= 0 || g.N <= 0 || g.K <= 0) throw std::runtime_error("sifter gemm: empty shape");
-    dim3 grid((g.N + kGBN - 1) / kGBN, (g.M + kGBM - 1) / kGBM);
-    if (ta == kF16 && tb == kBF16) gemm_kernel<__half, __nv_bfloat16><<<grid, 128, 0, s>>>(g);
-    else if (ta == kBF16 && tb == kBF16) gemm_kernel<__nv_bfloat16, __nv_bfloat16><<<grid, 128, 0, s>>>(g);
-    else if (ta == kF32 && tb == kBF16) gemm_kernel<float, __nv_bfloat16><<<grid, 128, 0, s>>>(g);
-    else if (ta == kF32 && tb == kF16) gemm_kernel<float, __half><<<grid, 128, 0, s>>>(g);
-    else throw std::runtime_error("sifter gemm: unsupported operand types");
-    sf_check_launch("gemm_kernel");
-}
-
-// ---------------------------------------------------------------------------------------------
-// Loss, elementwise and optimizer kernels.
-
-// Mean binary cross-entropy of the logits z against labels y; g[i] = (sigmoid(z_i) - y_i) / n.
-// One block of 1024 threads (n <= max_batch); loss[0] = mean loss.
-__global__ void __launch_bounds__(1024) bce_kernel(const float *z, const float *y, int n, float *g, float *loss)
-{
-    __shared__ float red[32];
-    float s = 0.0f;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const float zi = z[i], yi = y[i];
-        const float sig = 1.0f / (1.0f + expf(-zi));
-        g[i] = (sig - yi) / (float) n;
-        s += fmaxf(zi, 0.0f) - zi * yi + log1pf(expf(-fabsf(zi)));
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+#pragma unroll
+                for (int p = 0; p < 2; p++) {
+                    mma_bf16(acc[i][2 * p], a[i], b[p][0], b[p][1]);
+                    mma_bf16(acc[i][2 * p + 1], a[i], b[p][2], b[p][3]);
+                }
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        s = (threadIdx.x < (blockDim.x >> 5)) ? red[threadIdx.x] : 0.0f;
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (threadIdx.x == 0) loss[0] = s / (float) n;
-    }
-}
-
-// out = in * (z > 0), elementwise over count values.
-__global__ void relu_grad_kernel(const float *in, const float *z, float *out, long count)
-{
-    const long i = (long) blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < count) out[i] = (z[i] > 0.0f) ? in[i] : 0.0f;
-}
-
-// out[c] = sum_i g[i * H + c] (bias gradients).
-__global__ void colsum_kernel(const float *g, int n, int H, float *out)
-{
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= H) return;
-    float s = 0.0f;
-    for (int i = 0; i < n; i++) s += g[(long) i * H + c];
-    out[c] = s;
-}
-
-__global__ void adam_kernel(float *w, const float *g, float *m, float *v, long count, float lr, float c1, float c2)
-{
-    const long i = (long) blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const float gi = g[i];
-    const float mi = 0.9f * m[i] + 0.1f * gi;
-    const float vi = 0.999f * v[i] + 0.001f * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + 1.0e-8f);
+    const long o = first ? oW1 : oW2, ob = first ? bW1 : bW2;
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int t = 0; t < 4; t++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const long e = (long) (m0 + wm + i * 16 + (lane >> 2) + (q >> 1) * 8) * ldb + c0 + wn + t * 8 + (lane & 3) * 2 + (q & 1);
+                take_grad(g, o + e, ob + e, acc[i][t][q]);
+            }
 }
 
 __global__ void to_bf16_kernel(const float *src, uint16_t *dst, long count)
 {
     const long i = (long) blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
-    __nv_bfloat16 h = __float2bfloat16_rn(src[i]);
-    dst[i] = *(const uint16_t *) &h;
+    dst[i] = bf_bits(src[i]);
 }
 
 static unsigned blocks(long count, int t) { return (unsigned) ((count + t - 1) / t); }
 
 // ---------------------------------------------------------------------------------------------
-// Parameter layout.
-
-static constexpr long kW1 = long(kMlpH1) * kMlpIn, kB1 = kMlpH1, kW2 = long(kMlpH2) * kMlpH1, kB2 = kMlpH2, kW3 = kMlpH2, kB3 = 1;
-static constexpr long oW1 = 0, oB1 = oW1 + kW1, oW2 = oB1 + kB1, oB2 = oW2 + kW2, oW3 = oB2 + kB2, oB3 = oW3 + kW3;
-static constexpr long kNparams = oB3 + kB3;
-static constexpr long bW1 = 0, bW2 = kW1, bW3 = kW1 + kW2, kNbf16 = kW1 + kW2 + kW3;
 
 long Sifter::nparams() { return kNparams; }
 
@@ -315,14 +559,12 @@ Sifter::Sifter(int device_, long max_batch_, uint64_t seed) : device(device_), m
     SF_CHECK(cudaMalloc(&adam_v, kNparams * sizeof(float)));
     SF_CHECK(cudaMalloc(&wb, kNbf16 * sizeof(uint16_t)));
     SF_CHECK(cudaMalloc(&z1, max_batch * kMlpH1 * sizeof(float)));
-    SF_CHECK(cudaMalloc(&z2, max_batch * kMlpH2 * sizeof(float)));
-    SF_CHECK(cudaMalloc(&z3, max_batch * sizeof(float)));
-    SF_CHECK(cudaMalloc(&g, max_batch * sizeof(float)));
     SF_CHECK(cudaMalloc(&loss, sizeof(float)));
     SF_CHECK(cudaMalloc(&h1, max_batch * kMlpH1 * sizeof(uint16_t)));
-    SF_CHECK(cudaMalloc(&h2, max_batch * kMlpH2 * sizeof(uint16_t)));
-    SF_CHECK(cudaMalloc(&g1, max_batch * kMlpH1 * sizeof(float)));
-    SF_CHECK(cudaMalloc(&g2, max_batch * kMlpH2 * sizeof(float)));
+    SF_CHECK(cudaMalloc(&g1, max_batch * kMlpH1 * sizeof(uint16_t)));
+    SF_CHECK(cudaMalloc(&g2, max_batch * kMlpH2 * sizeof(uint16_t)));
+    SF_CHECK(cudaMalloc(&part, blocks(max_batch, kHeadRows) * kPart * sizeof(float)));
+    SF_CHECK(cudaFuncSetAttribute(head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(HeadSmem)));
     SF_CHECK(cudaMemset(adam_m, 0, kNparams * sizeof(float)));
     SF_CHECK(cudaMemset(adam_v, 0, kNparams * sizeof(float)));
     // He-uniform initial weights, zero biases.
@@ -332,25 +574,25 @@ Sifter::Sifter(int device_, long max_batch_, uint64_t seed) : device(device_), m
         std::uniform_real_distribution<double> u(-std::sqrt(6.0 / fan_in), std::sqrt(6.0 / fan_in));
         for (long i = 0; i < count; i++) p[off + i] = float(u(rng));
     };
-    fill(oW1, kW1, kMlpIn);
-    fill(oW2, kW2, kMlpH1);
-    fill(oW3, kW3, kMlpH2);
+    fill(oW1, kW1n, kMlpIn);
+    fill(oW2, kW2n, kMlpH1);
+    fill(oW3, kMlpH2, kMlpH2);
     set_params(p.data());
 }
 
 Sifter::~Sifter()
 {
     cudaSetDevice(device);
-    for (void *q : {(void *) master, (void *) grad, (void *) adam_m, (void *) adam_v, (void *) wb, (void *) z1, (void *) z2,
-                    (void *) z3, (void *) g, (void *) loss, (void *) h1, (void *) h2, (void *) g1, (void *) g2})
+    for (void *q : {(void *) master, (void *) grad, (void *) adam_m, (void *) adam_v, (void *) wb, (void *) z1,
+                    (void *) loss, (void *) h1, (void *) g1, (void *) g2, (void *) part})
         if (q) cudaFree(q);
 }
 
 void Sifter::refresh_bf16(cudaStream_t s)
 {
-    to_bf16_kernel<<<blocks(kW1, 256), 256, 0, s>>>(master + oW1, wb + bW1, kW1);
-    to_bf16_kernel<<<blocks(kW2, 256), 256, 0, s>>>(master + oW2, wb + bW2, kW2);
-    to_bf16_kernel<<<blocks(kW3, 256), 256, 0, s>>>(master + oW3, wb + bW3, kW3);
+    to_bf16_kernel<<<blocks(kW1n, 256), 256, 0, s>>>(master + oW1, wb + bW1, kW1n);
+    to_bf16_kernel<<<blocks(kW2n, 256), 256, 0, s>>>(master + oW2, wb + bW2, kW2n);
+    to_bf16_kernel<<<blocks(kMlpH2, 256), 256, 0, s>>>(master + oW3, wb + bW3, kMlpH2);
     sf_check_launch("to_bf16_kernel");
 }
 
@@ -368,86 +610,96 @@ void Sifter::get_params(float *host) const
     SF_CHECK(cudaMemcpy(host, master, kNparams * sizeof(float), cudaMemcpyDeviceToHost));
 }
 
+void Sifter::layer1(const uint16_t *patches, long n, cudaStream_t s)
+{
+    Layer1Args a;
+    a.x = patches;
+    a.w = wb + bW1;
+    a.bias = master + oB1;
+    a.n = int(n);
+    a.aligned = (reinterpret_cast<uintptr_t>(patches) & 15) == 0;   // a patch is 3456 bytes
+    a.z = z1;
+    a.h = h1;
+    // Split K until about one block per SM has work: the tiles are 32 x 32 of n x 256, 8 per 32 candidates, and a
+    // block's 27 K steps are a serial chain.
+    const long tiles = (kMlpH1 / 32) * blocks(n, 32);
+    const unsigned S = tiles <= 18 ? 8 : tiles <= 37 ? 4 : tiles <= 74 ? 2 : 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kMlpH1 / 32, blocks(n, 32), S);
+    cfg.blockDim = dim3(128);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = S;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    SF_CHECK(cudaLaunchKernelEx(&cfg, layer1_kernel, a));
+}
+
 void Sifter::forward(const uint16_t *patches, long n, float *logits, cudaStream_t s)
 {
     if (n < 1 || n > max_batch) throw std::runtime_error("Sifter::forward: batch size out of range");
     if (!patches || !logits) throw std::runtime_error("Sifter::forward: null pointer");
-    GemmArgs a;
-    memset(&a, 0, sizeof(a));
-    // Z1 = X W1^T + b1, H1 = bf16(relu(Z1))
-    a.M = int(n); a.N = kMlpH1; a.K = kMlpIn;
-    a.A = patches; a.sam = kMlpIn; a.sak = 1;
-    a.B = wb + bW1; a.sbn = kMlpIn; a.sbk = 1;
-    a.bias = master + oB1; a.relu = 1;
-    a.C = z1; a.ldc = kMlpH1; a.Cb = h1; a.ldcb = kMlpH1;
-    gemm(a, kF16, kBF16, s);
-    // Z2 = H1 W2^T + b2, H2 = bf16(relu(Z2))
-    a.N = kMlpH2; a.K = kMlpH1;
-    a.A = h1; a.sam = kMlpH1; a.sak = 1;
-    a.B = wb + bW2; a.sbn = kMlpH1; a.sbk = 1;
-    a.bias = master + oB2;
-    a.C = z2; a.ldc = kMlpH2; a.Cb = h2; a.ldcb = kMlpH2;
-    gemm(a, kBF16, kBF16, s);
-    // logit = H2 W3^T + b3
-    a.N = 1; a.K = kMlpH2;
-    a.A = h2; a.sam = kMlpH2; a.sak = 1;
-    a.B = wb + bW3; a.sbn = kMlpH2; a.sbk = 1;
-    a.bias = master + oB3; a.relu = 0;
-    a.C = logits; a.ldc = 1; a.Cb = nullptr;
-    gemm(a, kBF16, kBF16, s);
+    layer1(patches, n, s);
+    head(n, logits, nullptr, s);
 }
 
-// Gradients of the mean binary cross-entropy into 'grad' (after forward() into z3).
-void Sifter::backward(const uint16_t *patches, const float *labels, long n, cudaStream_t s)
+// Layers 2 and 3 of the batch in h1: the logits, or with labels the loss, g2, g1 and the partial gradients.
+void Sifter::head(long n, float *logits, const float *labels, cudaStream_t s)
 {
-    bce_kernel<<<1, 1024, 0, s>>>(z3, labels, int(n), g, loss);
-    sf_check_launch("bce_kernel");
-    GemmArgs a;
-    memset(&a, 0, sizeof(a));
-    // dW3 = g^T H2 (1 x 128)
-    a.M = 1; a.N = kMlpH2; a.K = int(n);
-    a.A = g; a.sam = 0; a.sak = 1;
-    a.B = h2; a.sbn = 1; a.sbk = kMlpH2;
-    a.C = grad + oW3; a.ldc = kMlpH2;
-    gemm(a, kF32, kBF16, s);
-    colsum_kernel<<<1, 32, 0, s>>>(g, int(n), 1, grad + oB3);
-    // gH2 = g W3 (n x 128), g2 = gH2 * (Z2 > 0)
-    a.M = int(n); a.N = kMlpH2; a.K = 1;
-    a.A = g; a.sam = 1; a.sak = 1;
-    a.B = wb + bW3; a.sbn = 1; a.sbk = kMlpH2;
-    a.C = g2; a.ldc = kMlpH2;
-    gemm(a, kF32, kBF16, s);
-    relu_grad_kernel<<<blocks(n * kMlpH2, 256), 256, 0, s>>>(g2, z2, g2, n * kMlpH2);
-    // dW2 = g2^T H1 (128 x 256), db2
-    a.M = kMlpH2; a.N = kMlpH1; a.K = int(n);
-    a.A = g2; a.sam = 1; a.sak = kMlpH2;
-    a.B = h1; a.sbn = 1; a.sbk = kMlpH1;
-    a.C = grad + oW2; a.ldc = kMlpH1;
-    gemm(a, kF32, kBF16, s);
-    colsum_kernel<<<blocks(kMlpH2, 128), 128, 0, s>>>(g2, int(n), kMlpH2, grad + oB2);
-    // gH1 = g2 W2 (n x 256), g1 = gH1 * (Z1 > 0)
-    a.M = int(n); a.N = kMlpH1; a.K = kMlpH2;
-    a.A = g2; a.sam = kMlpH2; a.sak = 1;
-    a.B = wb + bW2; a.sbn = 1; a.sbk = kMlpH1;
-    a.C = g1; a.ldc = kMlpH1;
-    gemm(a, kF32, kBF16, s);
-    relu_grad_kernel<<<blocks(n * kMlpH1, 256), 256, 0, s>>>(g1, z1, g1, n * kMlpH1);
-    // dW1 = g1^T X (256 x 1728), db1
-    a.M = kMlpH1; a.N = kMlpIn; a.K = int(n);
-    a.A = g1; a.sam = 1; a.sak = kMlpH1;
-    a.B = patches; a.sbn = 1; a.sbk = kMlpIn;
-    a.C = grad + oW1; a.ldc = kMlpIn;
-    gemm(a, kF32, kF16, s);
-    colsum_kernel<<<blocks(kMlpH1, 128), 128, 0, s>>>(g1, int(n), kMlpH1, grad + oB1);
-    sf_check_launch("sifter backward");
+    HeadArgs a;
+    a.h1 = h1;
+    a.w2 = wb + bW2;
+    a.w3 = wb + bW3;
+    a.z1 = z1;
+    a.b2 = master + oB2;
+    a.b3 = master + oB3;
+    a.n = int(n);
+    a.logits = logits;
+    a.labels = labels;
+    a.g1 = g1;
+    a.g2 = g2;
+    a.part = part;
+    head_kernel<<<blocks(n, kHeadRows), 256, sizeof(HeadSmem), s>>>(a);
+    sf_check_launch("head_kernel");
+}
+
+// Forward and backward of the mean binary cross-entropy: the gradients into 'grad', or one Adam step.
+void Sifter::train(const uint16_t *patches, const float *labels, long n, bool adam, float lr, cudaStream_t s)
+{
+    if (n < 1 || n > max_batch) throw std::runtime_error("Sifter::forward: batch size out of range");
+    if (!patches) throw std::runtime_error("Sifter::forward: null pointer");
+    layer1(patches, n, s);
+    head(n, nullptr, labels, s);
+    WgradArgs a;
+    a.g1 = g1;
+    a.g2 = g2;
+    a.h1 = h1;
+    a.x = patches;
+    a.part = part;
+    a.n = int(n);
+    a.nparts = int(blocks(n, kHeadRows));
+    a.aligned = (reinterpret_cast<uintptr_t>(patches) & 15) == 0;
+    a.loss = loss;
+    a.grad = adam ? nullptr : grad;
+    a.w = master;
+    a.m = adam_m;
+    a.v = adam_v;
+    a.wb = wb;
+    a.lr = lr;
+    a.c1 = 1.0f - std::pow(0.9f, float(step));
+    a.c2 = 1.0f - std::pow(0.999f, float(step));
+    wgrad_kernel<<<kWgTiles1 + kWgTiles2 + 1, 128, 0, s>>>(a);
+    sf_check_launch("wgrad_kernel");
 }
 
 double Sifter::gradients(const uint16_t *patches, const float *labels, long n, float *grad_host, cudaStream_t s)
 {
     if (!labels || !grad_host) throw std::runtime_error("Sifter::gradients: null pointer");
     SF_CHECK(cudaSetDevice(device));
-    forward(patches, n, z3, s);
-    backward(patches, labels, n, s);
+    train(patches, labels, n, false, 0.0f, s);
     float l = 0.0f;
     SF_CHECK(cudaMemcpyAsync(grad_host, grad, kNparams * sizeof(float), cudaMemcpyDeviceToHost, s));
     SF_CHECK(cudaMemcpyAsync(&l, loss, sizeof(float), cudaMemcpyDeviceToHost, s));
@@ -459,13 +711,8 @@ double Sifter::train_step(const uint16_t *patches, const float *labels, long n, 
 {
     if (!labels) throw std::runtime_error("Sifter::train_step: null pointer");
     SF_CHECK(cudaSetDevice(device));
-    forward(patches, n, z3, s);
-    backward(patches, labels, n, s);
-    step++;
-    const float c1 = 1.0f - std::pow(0.9f, float(step)), c2 = 1.0f - std::pow(0.999f, float(step));
-    adam_kernel<<<blocks(kNparams, 256), 256, 0, s>>>(master, grad, adam_m, adam_v, kNparams, lr, c1, c2);
-    sf_check_launch("adam_kernel");
-    refresh_bf16(s);
+    if (n >= 1 && n <= max_batch && patches) step++;
+    train(patches, labels, n, true, lr, s);
     float l = 0.0f;
     SF_CHECK(cudaMemcpyAsync(&l, loss, sizeof(float), cudaMemcpyDeviceToHost, s));
     SF_CHECK(cudaStreamSynchronize(s));

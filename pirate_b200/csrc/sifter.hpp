@@ -85,16 +85,19 @@ public:
     long max_batch = 0;
 
 private:
-    void backward(const uint16_t *patches, const float *labels, long n, cudaStream_t stream);
+    void layer1(const uint16_t *patches, long n, cudaStream_t stream);
+    void head(long n, float *logits, const float *labels, cudaStream_t stream);
+    void train(const uint16_t *patches, const float *labels, long n, bool adam, float lr, cudaStream_t stream);
     void refresh_bf16(cudaStream_t stream);
 
     float *master = nullptr;     // nparams fp32
     float *grad = nullptr;       // nparams fp32
     float *adam_m = nullptr, *adam_v = nullptr;
     uint16_t *wb = nullptr;      // bf16 copies of W1, W2, W3 (biases stay fp32)
-    float *z1 = nullptr, *z2 = nullptr, *z3 = nullptr, *g = nullptr, *loss = nullptr;
-    uint16_t *h1 = nullptr, *h2 = nullptr;   // bf16 activations
-    float *g2 = nullptr, *g1 = nullptr;
+    float *z1 = nullptr, *loss = nullptr;
+    uint16_t *h1 = nullptr;                  // bf16 activations
+    uint16_t *g2 = nullptr, *g1 = nullptr;   // bf16 gradients of Z2 and Z1 (as the products take them)
+    float *part = nullptr;                   // partial gradients of the biases and W3
     long step = 0;
 };
 
