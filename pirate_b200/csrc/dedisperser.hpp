@@ -239,8 +239,7 @@ private:
     bool sift = false;
     float sift_threshold = 0.0f;
     Sifter *sifter = nullptr;
-    DeviceBuffer d_cand, d_patches, d_peak_scratch;
-    int peak_split = 1;
+    DeviceBuffer d_cand, d_patches;
     PatchArgs patch_args;
     void *acquire_slot(long seq_id, cudaStream_t stream, void **int4);
 };

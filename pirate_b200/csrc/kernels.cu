@@ -13,6 +13,7 @@
 #include "kernels.cuh"
 #include "devutil.cuh"
 
+#include <cooperative_groups.h>
 #include <algorithm>
 #include <cstring>
 #include <stdexcept>
@@ -255,24 +256,35 @@ void launch_dequantize(void *out, int out_dtype, const void *data, const void *s
 }
 
 // ---------------------------------------------------------------------------------------------
-// Per-beam peak over a batch's outputs (the toy grouper's reduction, see BeamPeakArgs).
-// One 1024-thread block per beam scans every tree of that beam with 16-byte loads where the beam's
-// slice is aligned, keeping per thread the largest value and its first index; the block then
-// reduces with ties going to the smaller index, and thread 0 merges the trees in order.
+// Per-beam peak over a batch's outputs (the toy grouper's reduction, see BeamPeakArgs). The blocks of one cluster
+// share a beam: each scans its slice of every tree with 16-byte loads where the beam's data is aligned, keeping per
+// thread the largest value and its first index, and reduces them per tree; the first block then merges the slices
+// through distributed shared memory and the trees in order. One block per beam left the chip to as many SMs as
+// beams: 8 beams of a rank-16 plan (12.3 MB) took 44.7 us a call against 25.2 us, most of it the call's host part.
 
-// 16 bytes of out_max as raw words; element k of them as fp32.
+// Largest of the 16 bytes' elements (NaN if any is NaN), and element k, as fp32.
 template<typename T> struct PeakVec;
 template<> struct PeakVec<float>
 {
     static constexpr int N = 4;
-    __device__ static float get(const uint4 &q, int k)
+    __device__ static float max(const uint4 &q)
     {
-        return __uint_as_float(k == 0 ? q.x : k == 1 ? q.y : k == 2 ? q.z : q.w);
+        float m;
+        asm("{.reg .f32 a, b;\n max.NaN.f32 a, %1, %2;\n max.NaN.f32 b, %3, %4;\n max.NaN.f32 %0, a, b;}"
+            : "=f"(m) : "f"(__uint_as_float(q.x)), "f"(__uint_as_float(q.y)), "f"(__uint_as_float(q.z)), "f"(__uint_as_float(q.w)));
+        return m;
     }
+    __device__ static float get(const uint4 &q, int k) { return __uint_as_float(k == 0 ? q.x : k == 1 ? q.y : k == 2 ? q.z : q.w); }
 };
 template<> struct PeakVec<__half>
 {
     static constexpr int N = 8;
+    __device__ static float max(const uint4 &q)
+    {
+        const __half2 m = __hmax2_nan(__hmax2_nan(*(const __half2 *) &q.x, *(const __half2 *) &q.y),
+                                      __hmax2_nan(*(const __half2 *) &q.z, *(const __half2 *) &q.w));
+        return __half2float(__hmax_nan(__low2half(m), __high2half(m)));
+    }
     __device__ static float get(const uint4 &q, int k)
     {
         const uint32_t w = (k < 2) ? q.x : (k < 4) ? q.y : (k < 6) ? q.z : q.w;
@@ -282,6 +294,12 @@ template<> struct PeakVec<__half>
 template<> struct PeakVec<__nv_bfloat16>
 {
     static constexpr int N = 8;
+    __device__ static float max(const uint4 &q)
+    {
+        const __nv_bfloat162 m = __hmax2_nan(__hmax2_nan(*(const __nv_bfloat162 *) &q.x, *(const __nv_bfloat162 *) &q.y),
+                                             __hmax2_nan(*(const __nv_bfloat162 *) &q.z, *(const __nv_bfloat162 *) &q.w));
+        return __bfloat162float(__hmax_nan(__low2bfloat16(m), __high2bfloat16(m)));
+    }
     __device__ static float get(const uint4 &q, int k)
     {
         const uint32_t w = (k < 2) ? q.x : (k < 4) ? q.y : (k < 6) ? q.z : q.w;
@@ -289,190 +307,112 @@ template<> struct PeakVec<__nv_bfloat16>
     }
 };
 
-__device__ __forceinline__ void peak_take(float v, long i, float &bv, long &bi)
+// A slice's maximum and its first index; v is NaN where the slice holds a NaN.
+struct PeakPart
 {
-    if (v > bv || (v == bv && i < bi)) { bv = v; bi = i; }
+    float v;
+    int i;
+};
+constexpr int kPeakNone = 0x7fffffff;
+
+// The larger, on a tie the smaller index; NaN if either is.
+__device__ __forceinline__ PeakPart peak_merge(PeakPart a, PeakPart b)
+{
+    if (a.v != a.v) return a;
+    if (b.v != b.v) return b;
+    return (b.v > a.v || (b.v == a.v && b.i < a.i)) ? b : a;
+}
+
+__device__ __forceinline__ PeakPart peak_warp(PeakPart p)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        PeakPart q;
+        q.v = __shfl_xor_sync(0xffffffffu, p.v, o);
+        q.i = __shfl_xor_sync(0xffffffffu, p.i, o);
+        p = peak_merge(p, q);
+    }
+    return p;
 }
 
 template<typename T>
 __global__ void __launch_bounds__(1024) beam_peak_kernel(BeamPeakArgs a)
 {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
     constexpr int V = PeakVec<T>::N;
-    constexpr long kNone = 0x7fffffffffffffffL;
-    __shared__ float rv[32];
-    __shared__ long ri[32];
-    __shared__ int rn[32];
-    const int b = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ PeakPart wp[kBeamPeakMaxTrees][32];   // per tree and warp; in the first block, per tree the merged slices
+    __shared__ PeakPart bp[kBeamPeakMaxTrees];       // per tree, this block's slice
+    const int C = int(cl.num_blocks()), rank = int(cl.block_rank());
+    const int b = blockIdx.x / C, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nwarps = blockDim.x >> 5;
-
-    float gv = -INFINITY;            // thread 0: best over the trees so far
-    int gt = -1;
-    long gi = 0;
 
     for (int t = 0; t < a.ntrees; t++) {
         const long n = a.ndm[t] * a.nt[t];
         const T *x = (const T *) a.out_max[t] + (long) b * n;
-        float bv = -INFINITY;
-        long bi = kNone;
+        PeakPart p = {-INFINITY, kPeakNone};
         bool nan = false;
         if (n % V == 0 && ((uintptr_t) x & 15) == 0) {
-            const long nv = n / V;
+            const long nv = n / V, per = (nv + C - 1) / C;
+            const long lo = rank * per, hi = min(nv, lo + per);
             const uint4 *xv = (const uint4 *) x;
-            for (long j = threadIdx.x; j < nv; j += 4L * blockDim.x) {
+            for (long j = lo + threadIdx.x; j < hi; j += 4L * blockDim.x) {
                 uint4 q[4];
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
                     const long jj = j + (long) u * blockDim.x;
-                    if (jj < nv) q[u] = __ldg(xv + jj);
+                    if (jj < hi) q[u] = __ldg(xv + jj);
                 }
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
                     const long jj = j + (long) u * blockDim.x;
-                    if (jj < nv) {
+                    if (jj < hi) {
+                        const float m = PeakVec<T>::max(q[u]);
+                        nan |= (m != m);
+                        if (m > p.v) {
+                            p.v = m;
 #pragma unroll
-                        for (int k = 0; k < V; k++) {
-                            const float v = PeakVec<T>::get(q[u], k);
-                            nan |= (v != v);
-                            if (v > bv) { bv = v; bi = jj * V + k; }
+                            for (int k = V - 1; k >= 0; k--)
+                                if (PeakVec<T>::get(q[u], k) == m) p.i = int(jj * V) + k;
                         }
                     }
                 }
             }
         } else {
-            for (long i = threadIdx.x; i < n; i += blockDim.x) {
+            const long per = (n + C - 1) / C, lo = rank * per, hi = min(n, lo + per);
+            for (long i = lo + threadIdx.x; i < hi; i += blockDim.x) {
                 const float v = to_f(x[i]);
                 nan |= (v != v);
-                if (v > bv) { bv = v; bi = i; }
+                if (v > p.v) { p.v = v; p.i = int(i); }
             }
         }
-
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            peak_take(__shfl_down_sync(0xffffffffu, bv, o), __shfl_down_sync(0xffffffffu, bi, o), bv, bi);
-        const bool wnan = __any_sync(0xffffffffu, nan);
-        if (lane == 0) { rv[warp] = bv; ri[warp] = bi; rn[warp] = wnan; }
-        __syncthreads();
-        if (warp == 0) {
-            bv = (lane < nwarps) ? rv[lane] : -INFINITY;
-            bi = (lane < nwarps) ? ri[lane] : kNone;
-            const bool tnan = __any_sync(0xffffffffu, (lane < nwarps) && rn[lane]);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-                peak_take(__shfl_down_sync(0xffffffffu, bv, o), __shfl_down_sync(0xffffffffu, bi, o), bv, bi);
-            if (lane == 0 && !tnan && bv > gv) { gv = bv; gt = t; gi = bi; }
-        }
-        __syncthreads();
+        if (nan) p.v = NAN;
+        p = peak_warp(p);
+        if (lane == 0) wp[t][warp] = p;
     }
-
-    if (threadIdx.x == 0) {
-        a.peak[b] = gv;
-        a.tree[b] = gt;
-        if (gt >= 0) {
-            const long nt = a.nt[gt];
-            a.idm[b] = int(gi / nt);
-            a.itime[b] = int(gi % nt);
-            a.token[b] = a.out_argmax[gt][(long) b * a.ndm[gt] * nt + gi];
-        } else {
-            a.idm[b] = -1;
-            a.itime[b] = -1;
-            a.token[b] = 0;
-        }
-    }
-}
-
-struct PeakPartial
-{
-    float v;      // maximum of the slice (-inf if empty)
-    int nan;      // the slice holds a NaN
-    long i;       // first position of the maximum in the tree (kNone if none)
-};
-
-// Grid (nsplit, ntrees, nbeams): block (s, t, b) reduces slice s of tree t of beam b.
-template<typename T>
-__global__ void __launch_bounds__(256) beam_peak_split_kernel(BeamPeakArgs a, PeakPartial *part, int nsplit)
-{
-    constexpr int V = PeakVec<T>::N;
-    constexpr long kNone = 0x7fffffffffffffffL;
-    __shared__ float rv[8];
-    __shared__ long ri[8];
-    __shared__ int rn[8];
-    const int s = blockIdx.x, t = blockIdx.y, b = blockIdx.z;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long n = a.ndm[t] * a.nt[t];
-    const T *x = (const T *) a.out_max[t] + (long) b * n;
-    float bv = -INFINITY;
-    long bi = kNone;
-    bool nan = false;
-    if (n % V == 0 && ((uintptr_t) x & 15) == 0) {
-        const long nv = n / V, per = (nv + nsplit - 1) / nsplit;
-        const long lo = (long) s * per, hi = min(nv, lo + per);
-        const uint4 *xv = (const uint4 *) x;
-        for (long j = lo + threadIdx.x; j < hi; j += blockDim.x) {
-            const uint4 q = __ldg(xv + j);
-#pragma unroll
-            for (int k = 0; k < V; k++) {
-                const float v = PeakVec<T>::get(q, k);
-                nan |= (v != v);
-                if (v > bv) { bv = v; bi = j * V + k; }
-            }
-        }
-    } else {
-        const long per = (n + nsplit - 1) / nsplit;
-        const long lo = (long) s * per, hi = min(n, lo + per);
-        for (long i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-            const float v = to_f(x[i]);
-            nan |= (v != v);
-            if (v > bv) { bv = v; bi = i; }
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        peak_take(__shfl_down_sync(0xffffffffu, bv, o), __shfl_down_sync(0xffffffffu, bi, o), bv, bi);
-    const bool wnan = __any_sync(0xffffffffu, nan);
-    if (lane == 0) { rv[warp] = bv; ri[warp] = bi; rn[warp] = wnan; }
     __syncthreads();
-    if (warp == 0) {
-        const int nw = blockDim.x >> 5;
-        bv = (lane < nw) ? rv[lane] : -INFINITY;
-        bi = (lane < nw) ? ri[lane] : kNone;
-        const bool tn = __any_sync(0xffffffffu, (lane < nw) && rn[lane]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            peak_take(__shfl_down_sync(0xffffffffu, bv, o), __shfl_down_sync(0xffffffffu, bi, o), bv, bi);
-        if (lane == 0) {
-            PeakPartial &p = part[((long) b * a.ntrees + t) * nsplit + s];
-            p.v = bv;
-            p.nan = tn ? 1 : 0;
-            p.i = bi;
+    for (int t = warp; t < a.ntrees; t += nwarps) {
+        PeakPart p = {-INFINITY, kPeakNone};
+        if (lane < nwarps) p = wp[t][lane];
+        p = peak_warp(p);
+        if (lane == 0) bp[t] = p;
+    }
+    cl.sync();
+    if (rank == 0) {
+        for (int t = warp; t < a.ntrees; t += nwarps) {
+            PeakPart p = {-INFINITY, kPeakNone};
+            if (lane < C) p = cl.map_shared_rank(bp, lane)[t];
+            p = peak_warp(p);
+            if (lane == 0) wp[t][0] = p;
         }
     }
-}
-
-// One warp per beam: per tree (in order) the slices' maximum with the first position, a tree holding a
-// NaN passed over, then the first tree with the strictly largest maximum (beam_peak_kernel's rules).
-__global__ void beam_peak_final_kernel(BeamPeakArgs a, const PeakPartial *part, int nsplit)
-{
-    constexpr long kNone = 0x7fffffffffffffffL;
-    const int b = blockIdx.x, lane = threadIdx.x;
-    float gv = -INFINITY;
-    int gt = -1;
-    long gi = 0;
-    for (int t = 0; t < a.ntrees; t++) {
-        float bv = -INFINITY;
-        long bi = kNone;
-        bool nan = false;
-        for (int s = lane; s < nsplit; s += 32) {
-            const PeakPartial p = part[((long) b * a.ntrees + t) * nsplit + s];
-            nan |= (p.nan != 0);
-            peak_take(p.v, p.i, bv, bi);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            peak_take(__shfl_down_sync(0xffffffffu, bv, o), __shfl_down_sync(0xffffffffu, bi, o), bv, bi);
-        const bool tnan = __any_sync(0xffffffffu, nan);
-        if (lane == 0 && !tnan && bv > gv) { gv = bv; gt = t; gi = bi; }
-    }
-    if (lane == 0) {
+    cl.sync();   // every slice has been read
+    if (rank == 0 && threadIdx.x == 0) {
+        // The first tree with the strictly largest maximum; a tree holding a NaN is passed over.
+        float gv = -INFINITY;
+        int gt = -1, gi = 0;
+        for (int t = 0; t < a.ntrees; t++)
+            if (wp[t][0].v > gv) { gv = wp[t][0].v; gt = t; gi = wp[t][0].i; }
         a.peak[b] = gv;
         a.tree[b] = gt;
         if (gt >= 0) {
@@ -486,23 +426,6 @@ __global__ void beam_peak_final_kernel(BeamPeakArgs a, const PeakPartial *part, 
             a.token[b] = 0;
         }
     }
-}
-
-void launch_beam_peaks_split(const BeamPeakArgs &a, int dtype, long nbeams, void *scratch, int nsplit, cudaStream_t s)
-{
-    if (a.ntrees <= 0 || a.ntrees > kBeamPeakMaxTrees) throw std::runtime_error("beam_peaks: bad number of trees");
-    if (!scratch || nsplit < 1 || nsplit > 1024) throw std::runtime_error("beam_peaks: bad split scratch");
-    if (nbeams <= 0) return;
-    if (nbeams > 65535) throw std::runtime_error("beam_peaks: too many beams for the split reduction");
-    dim3 grid((unsigned) nsplit, (unsigned) a.ntrees, (unsigned) nbeams);
-    PeakPartial *part = (PeakPartial *) scratch;
-    if (dtype == 0) beam_peak_split_kernel<float><<<grid, 256, 0, s>>>(a, part, nsplit);
-    else if (dtype == 1) beam_peak_split_kernel<__half><<<grid, 256, 0, s>>>(a, part, nsplit);
-    else if (dtype == 2) beam_peak_split_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(a, part, nsplit);
-    else throw std::runtime_error("beam_peaks: bad dtype");
-    check_launch("beam_peak_split_kernel");
-    beam_peak_final_kernel<<<(unsigned) nbeams, 32, 0, s>>>(a, part, nsplit);
-    check_launch("beam_peak_final_kernel");
 }
 
 void launch_beam_peaks(const BeamPeakArgs &a, int dtype, long nbeams, cudaStream_t s)
@@ -516,12 +439,26 @@ void launch_beam_peaks(const BeamPeakArgs &a, int dtype, long nbeams, cudaStream
     }
     if (nbeams <= 0) return;
     if (nbeams > 0x7fffffffL) throw std::runtime_error("beam_peaks: too many beams");
-    const unsigned grid = (unsigned) nbeams;
-    if (dtype == 0) beam_peak_kernel<float><<<grid, 1024, 0, s>>>(a);
-    else if (dtype == 1) beam_peak_kernel<__half><<<grid, 1024, 0, s>>>(a);
-    else if (dtype == 2) beam_peak_kernel<__nv_bfloat16><<<grid, 1024, 0, s>>>(a);
+    // Blocks per beam: up to 8 (the portable cluster size), about two per SM over all beams.
+    unsigned C = 8;
+    while (C > 1 && nbeams * C > 2 * 148) C /= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned) nbeams * C);
+    cfg.blockDim = dim3(1024);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaError_t e;
+    if (dtype == 0) e = cudaLaunchKernelEx(&cfg, beam_peak_kernel<float>, a);
+    else if (dtype == 1) e = cudaLaunchKernelEx(&cfg, beam_peak_kernel<__half>, a);
+    else if (dtype == 2) e = cudaLaunchKernelEx(&cfg, beam_peak_kernel<__nv_bfloat16>, a);
     else throw std::runtime_error("beam_peaks: dtype must be 0 (float32), 1 (float16) or 2 (bfloat16)");
-    check_launch("beam_peak_kernel");
+    if (e != cudaSuccess) throw std::runtime_error(std::string("beam_peak_kernel: ") + cudaGetErrorString(e));
 }
 
 // ---------------------------------------------------------------------------------------------
