@@ -223,19 +223,45 @@ __device__ __forceinline__ void grid_run_lut(const GridLdsArgs &a, int b, int f0
     }
 }
 
-// Standalone dequantization: one thread per 32 samples (16 input bytes, 16-byte output stores).
+// Standalone dequantization, bound by HBM. A thread turns 16 output bytes' worth of samples at a time, so that a
+// warp's loads and stores are each one contiguous run, four of them a block apart in flight. Rows are multiples of
+// 256 samples and contiguous, so sample, scale block and byte offsets are the flat index's. (One thread per 32
+// samples stored 16 bytes per lane 64 bytes apart: 81.7 us for 4 x 16384 x 2048 samples to fp16, against 67.5 us, 5.0 TB/s.)
+constexpr int kDequantUnroll = 4;
+
 template<typename To>
-__global__ void __launch_bounds__(256) dequant_kernel(To *out, const uint8_t *data, const __half2 *scoff, long rows, int T)
+__global__ void __launch_bounds__(256) dequant_kernel(To *out, const uint8_t *data, const __half2 *scoff, long units)
 {
-    const long nper = T / 32;
-    const long g = (long) blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= rows * nper)
-        return;
-    const long row = g / nper;
-    const long t0 = (g - row * nper) * 32;
-    float o[32];
-    load_run_q<To, 32>(data + row * (T >> 1), scoff + row * (T >> 8), t0, o);
-    store_run<To, 32>(out + row * T + t0, o);
+    constexpr int SPT = 16 / sizeof(To);   // 4 or 8 samples
+    using In = typename std::conditional<SPT == 8, uint32_t, uint16_t>::type;
+    const long u0 = (long) blockIdx.x * (256 * kDequantUnroll) + threadIdx.x;
+    In w[kDequantUnroll];
+    float2 so[kDequantUnroll];
+#pragma unroll
+    for (int k = 0; k < kDequantUnroll; k++) {
+        const long u = u0 + 256 * k;
+        if (u < units) {
+            w[k] = __ldg((const In *) data + u);
+            so[k] = __half22float2(__ldg(scoff + (u * SPT >> 8)));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kDequantUnroll; k++) {
+        const long u = u0 + 256 * k;
+        if (u < units) {
+            float o[SPT];
+#pragma unroll
+            for (int i = 0; i < SPT; i++) o[i] = dq_value(uint32_t(w[k]) >> (4 * i), so[k].x, so[k].y);
+            store_run<To, SPT>(out + u * SPT, o);
+        }
+    }
+}
+
+template<typename To>
+static void launch_dequant_t(void *out, const void *data, const void *scoff, long samples, cudaStream_t s)
+{
+    const long units = samples / (16 / long(sizeof(To))), grid = (units + 256 * kDequantUnroll - 1) / (256 * kDequantUnroll);
+    dequant_kernel<To><<<(unsigned) grid, 256, 0, s>>>((To *) out, (const uint8_t *) data, (const __half2 *) scoff, units);
 }
 
 void launch_dequantize(void *out, int out_dtype, const void *data, const void *scales_offsets, long nbeams, long nfreq,
@@ -243,15 +269,11 @@ void launch_dequantize(void *out, int out_dtype, const void *data, const void *s
 {
     if (ntime <= 0 || ntime % 256) throw std::runtime_error("dequantize: ntime must be a positive multiple of 256");
     if (!out || !data || !scales_offsets) throw std::runtime_error("dequantize: null pointer");
-    const long rows = nbeams * nfreq;
-    const long nthr = rows * (ntime / 32);
-    if (nthr == 0) return;
-    const unsigned grid = (unsigned) ((nthr + 255) / 256);
-    const uint8_t *d = (const uint8_t *) data;
-    const __half2 *so = (const __half2 *) scales_offsets;
-    if (out_dtype == 0) dequant_kernel<float><<<grid, 256, 0, s>>>((float *) out, d, so, rows, int(ntime));
-    else if (out_dtype == 1) dequant_kernel<__half><<<grid, 256, 0, s>>>((__half *) out, d, so, rows, int(ntime));
-    else dequant_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((__nv_bfloat16 *) out, d, so, rows, int(ntime));
+    const long samples = nbeams * nfreq * ntime;
+    if (samples == 0) return;
+    if (out_dtype == 0) launch_dequant_t<float>(out, data, scales_offsets, samples, s);
+    else if (out_dtype == 1) launch_dequant_t<__half>(out, data, scales_offsets, samples, s);
+    else launch_dequant_t<__nv_bfloat16>(out, data, scales_offsets, samples, s);
     check_launch("dequant_kernel");
 }
 
