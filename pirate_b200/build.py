@@ -14,8 +14,8 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libpirate_b200.so")
 
-SOURCES = ["plan.cpp", "avar.cpp", "simpulse.cpp", "capi.cpp", "kernels.cu", "tree_halo_f32.cu", "tree_halo_f16.cu", "tree_halo_bf16.cu", "dedisperser.cu", "noalloc.cu", "sifter.cu", "batched.cu"]
-HEADERS = ["plan.hpp", "avar.hpp", "simpulse.hpp", "yaml_lite.hpp", "kernels.cuh", "devutil.cuh", "tree_halo.cuh", "tree_halo_kernel.cuh", "dedisperser.hpp", "regtree.cuh", "sifter.hpp", "batched.hpp"]
+SOURCES = ["plan.cpp", "avar.cpp", "simpulse.cpp", "capi.cpp", "kernels.cu", "tree_halo_f32.cu", "tree_halo_f16.cu", "tree_halo_bf16.cu", "pf_reg_f32.cu", "pf_reg_f16.cu", "pf_reg_bf16.cu", "dedisperser.cu", "noalloc.cu", "sifter.cu", "batched.cu"]
+HEADERS = ["plan.hpp", "avar.hpp", "simpulse.hpp", "yaml_lite.hpp", "kernels.cuh", "devutil.cuh", "tree_halo.cuh", "tree_halo_kernel.cuh", "pf_reg.cuh", "dedisperser.hpp", "regtree.cuh", "sifter.hpp", "batched.hpp"]
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

@@ -22,33 +22,6 @@
 
 namespace pb2 {
 
-// Two fp32 additions (multiplications) in one sm_100 packed f32x2 instruction; each element is
-// rounded to nearest like __fadd_rn (__fmul_rn).
-__device__ __forceinline__ unsigned long long f2pack(float2 a)
-{
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
-    return r;
-}
-__device__ __forceinline__ float2 f2unpack(unsigned long long r)
-{
-    float2 d;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(r));
-    return d;
-}
-__device__ __forceinline__ float2 f2add(float2 a, float2 b)
-{
-    unsigned long long d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(f2pack(a)), "l"(f2pack(b)));
-    return f2unpack(d);
-}
-__device__ __forceinline__ float2 f2mul(float2 a, float2 b)
-{
-    unsigned long long d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(f2pack(a)), "l"(f2pack(b)));
-    return f2unpack(d);
-}
-
 // -------------------------------------------------------------------------------------------------
 // Tree gridding fused with lagged downsampling.
 //
@@ -696,10 +669,7 @@ __global__ void __launch_bounds__(kGridMaxThreads) grid_lds_kernel(GridLdsArgs a
 // each lane then scans the trials of its output time. The running maximum breaks ties by the
 // reference's scan order (level, multiplet, fine time, profile), reproducing its out_argmax tokens.
 
-
 constexpr int kPfWarps = 4;
-constexpr int kPfMaxLevels = 6;
-constexpr int kPfMaxProfiles = 16;   // 1 + 3 log2(max_width), max_width <= 32
 
 // Number of entries of boxcar level l in a window of len0 samples (level 0 = samples).
 __device__ __forceinline__ int pf_nlev(int len0, int l, int dt) { return (len0 - (1 << l)) / dt + 1; }
@@ -851,466 +821,6 @@ __global__ void __launch_bounds__(kPfWarps * 32) pf_kernel(PfArgs a, int warp_fl
 
 
 // -------------------------------------------------------------------------------------------------
-// Fast peak finding (output time downsampling Dout >= 4; the general kernel above covers the rest).
-//
-// Same work split (one warp per beam, coarse dm and 32 output times; lane = output time) and the same
-// results, organised around four changes:
-//
-//  1. Bank-conflict-free shared memory. Level l of the boxcar window is stored in blocks of nsamp_l
-//     entries (one block per lane: its output time's fine samples). Levels scanned in pairs with
-//     blocks of >= 4 entries pad each block with 2 floats, so the 32 blocks fall on distinct banks
-//     for 8-byte loads; the other levels are contiguous and are read in pairs or single floats.
-//  2. Levels are built while they are scanned: while a lane scans its fine samples at level l two at
-//     a time, the pair's sum is its level-(l+1) entry (B_{l+1}[u] = B_l[2u] + B_l[2u+1] while
-//     dt doubles), so only the pad region before the first output time and the levels with
-//     saturated time step (dt = Dcore) are built in a separate pass.
-//  3. Max-only trial loop. The scan keeps, per group (level, multiplet), the maximum trial value
-//     (fmaxf and the three-input max, which ignore NaN as the reference's strict '>' does) and the
-//     first fine sample (pair) reaching it; across groups, the first group in the reference's
-//     (level, multiplet) order whose maximum equals the overall one. After each multiplet, a lane
-//     whose maximum moved into it recomputes that fine sample's (pair's) trials from shared memory
-//     and takes the first, in (fine time, profile) order, equal to the maximum: its value and token
-//     are the outputs.
-//  4. The next multiplet's window is staged in shared memory with cp.async while the current one is
-//     scanned.
-
-// Per-level constants of the fast peak finder (host-computed; level l has time step dt, boxcar
-// length 2^l = S*dt, and nsamp = Dout/dt fine samples per output time).
-enum { kPfU = 1, kPfPairs = 2, kPfNextU = 4 };
-struct PfGeom
-{
-    int off[kPfMaxLevels];   // first float of level l in a warp's region (even)
-    int e[kPfMaxLevels];     // entry i lies in block (i + e) >> k
-    int k[kPfMaxLevels];     // log2(nsamp_l)
-    int pad[kPfMaxLevels];   // floats after each block
-    int I[kPfMaxLevels];     // entry of the warp's first output time's first fine sample
-    int n[kPfMaxLevels];     // entries of level l in the window of 32 output times
-    int dt[kPfMaxLevels], S[kPfMaxLevels], nsamp[kPfMaxLevels];
-    int rr[kPfMaxLevels], ss[kPfMaxLevels];   // B_l[u] = B_{l-1}[rr u] + B_{l-1}[rr u + ss]
-    int flags[kPfMaxLevels]; // kPfU: dt = 2^l; kPfPairs: scanned two fine samples at a time;
-                             // kPfNextU: level l+1 has dt = 2^(l+1) and is built by this level's scan
-    int raw_off;             // two staging buffers of the window's raw samples (16-byte aligned), one per
-    int raw_floats;          // multiplet in flight, raw_floats apart; level 0 is read from them directly
-    int w_off;               // the warp's weights of one subband, [profile < 16][weight time < 32]
-    int warp_floats;
-};
-
-// max(a, b, c) ignoring NaN inputs (sm_100 three-input max).
-__device__ __forceinline__ float pf_max3(float a, float b, float c)
-{
-    float d;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
-
-__device__ __forceinline__ int pf_phys(const PfGeom &g, int l, int i)
-{
-    const int t = i + g.e[l];
-    return g.off[l] + t + g.pad[l] * (t >> g.k[l]);
-}
-
-template<typename Ts> __device__ __forceinline__ void pf_load4(const Ts *p, float (&v)[4]);
-template<> __device__ __forceinline__ void pf_load4<float>(const float *p, float (&v)[4])
-{
-    const float4 q = *(const float4 *) p;
-    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-}
-template<> __device__ __forceinline__ void pf_load4<__half>(const __half *p, float (&v)[4])
-{
-    const uint2 q = *(const uint2 *) p;
-    const float2 a = __half22float2(*(const __half2 *) &q.x), b = __half22float2(*(const __half2 *) &q.y);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-template<> __device__ __forceinline__ void pf_load4<__nv_bfloat16>(const __nv_bfloat16 *p, float (&v)[4])
-{
-    const uint2 q = *(const uint2 *) p;
-    const float2 a = __bfloat1622float2(*(const __nv_bfloat162 *) &q.x), b = __bfloat1622float2(*(const __nv_bfloat162 *) &q.y);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-// Eight samples from a 16-byte-aligned address (two 4-sample loads for fp32).
-template<typename Ts> __device__ __forceinline__ void pf_load8(const Ts *p, float (&v)[8])
-{
-    if constexpr (sizeof(Ts) == 4) {
-        float a[4], b[4];
-        pf_load4<Ts>(p, a);
-        pf_load4<Ts>(p + 4, b);
-#pragma unroll
-        for (int i = 0; i < 4; i++) { v[i] = a[i]; v[4 + i] = b[i]; }
-    } else {
-        const uint4 q = *(const uint4 *) p;
-        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            float2 f;
-            if constexpr (std::is_same<Ts, __half>::value) f = __half22float2(*(const __half2 *) &w[i]);
-            else f = __bfloat1622float2(*(const __nv_bfloat162 *) &w[i]);
-            v[2 * i] = f.x; v[2 * i + 1] = f.y;
-        }
-    }
-}
-
-// Shared-memory layout of the fast peak finder for one warp (see PfGeom).
-// LW: output times (lanes) per coarse DM in a warp (32, or 16 and 8 for trees with that few output
-// times per chunk: 32 / LW coarse DMs then share a warp).
-__host__ __device__ constexpr PfGeom pf_geom(int Dout, int Dcore, int tpad, int L, int esize, int LW = 32)
-{
-    PfGeom g{};
-    int off = 0;
-    for (int l = 0; l < L; l++) {
-        const int dt = (Dcore < (1 << l)) ? Dcore : (1 << l);
-        const int nsamp = Dout / dt;
-        const bool pairs = ((1 << l) <= Dcore) && nsamp >= 2;
-        const int I = (tpad + dt - (1 << l)) / dt;
-        int k = 0;
-        while ((1 << k) < nsamp) k++;
-        g.off[l] = off;
-        g.e[l] = (nsamp - I % nsamp) % nsamp;
-        g.k[l] = k;
-        // Levels scanned in pairs from per-lane blocks: 2 floats after each block of >= 4 (the
-        // blocks then fall on distinct banks for 8-byte loads); the others are stored contiguously.
-        g.pad[l] = (pairs && nsamp >= 4) ? 2 : 0;
-        g.I[l] = I;
-        g.n[l] = LW * nsamp + I;
-        g.dt[l] = dt;
-        g.S[l] = (1 << l) / dt;
-        g.nsamp[l] = nsamp;
-        if (l > 0) {
-            const int dtp = (Dcore < (1 << (l - 1))) ? Dcore : (1 << (l - 1));
-            g.rr[l] = dt / dtp;
-            g.ss[l] = (1 << (l - 1)) / dtp;
-        }
-        g.flags[l] = (((1 << l) <= Dcore) ? kPfU : 0) | (pairs ? kPfPairs : 0)
-                   | ((l + 1 < L && (2 << l) <= Dcore) ? kPfNextU : 0);
-        const int t = g.n[l] - 1 + g.e[l];
-        const int size = t + g.pad[l] * (t >> k) + 1;
-        if (l > 0)   // level 0 lives only in the raw staging buffer
-            off += (size + 1) & ~1;
-    }
-    g.raw_off = (off + 3) & ~3;
-    g.raw_floats = ((LW * Dout + tpad) * esize + 15) / 16 * 4;
-    g.w_off = g.raw_off + 2 * g.raw_floats;
-    g.warp_floats = g.w_off + kPfMaxProfiles * 32;
-    return g;
-}
-
-// Peak-finder constants fixed by the plan rules: Dcore = min(Dout, 8) and tpad = max(2 Wmax, 4) with
-// L = max(log2 Wmax, 1), i.e. tpad = max(2^(L+1), 4).
-__host__ __device__ constexpr int pf_dcore_of(int Dout) { return Dout < 8 ? Dout : 8; }
-__host__ __device__ constexpr int pf_tpad_of(int L) { return (2 << L) > 4 ? (2 << L) : 4; }
-
-// The kernel body. g holds the per-level constants (a compile-time constant object when DOUT > 0, so
-// the unrolled level loop sees them as immediates); gr is the same geometry passed at launch, used
-// where the level is only known at run time.
-// CTR: the chunk index comes from the device counter (replayed CUDA graphs). It is a template flag
-// because reading it costs the kernel about 26 registers, which the direct launches should not pay.
-template<typename Ts, int L, int DOUT, bool CTR, int LW>
-__device__ __forceinline__ void pf_fast_body(const PfArgs &a, const PfGeom &g, const PfGeom &gr)
-{
-    static_assert(LW == 32 || LW == 16 || LW == 8, "lanes per coarse DM");
-    constexpr int G = 32 / LW;   // coarse DMs per warp, each on LW consecutive lanes
-    extern __shared__ float sm[];
-    const int warp = threadIdx.x >> 5, sub = (threadIdx.x & 31) / LW, lane = threadIdx.x & (LW - 1);
-    const int dm0 = (blockIdx.y * kPfWarps + warp) * G;
-    const int b = blockIdx.z, bt = a.beam0 + b;
-    const int tout0 = blockIdx.x * LW;
-    if (dm0 >= a.ndm_out)
-        return;   // whole warp exits; warps never synchronize across the block
-    // A sub-group past the last coarse DM computes the last one again and stores nothing.
-    const bool dm_ok = dm0 + sub < a.ndm_out;
-    const int dm = dm_ok ? dm0 + sub : a.ndm_out - 1;
-
-    const int ntw = min(LW, a.nt_out - tout0);
-    const int tout = tout0 + lane;
-    const bool active = (lane < ntw) && dm_ok;
-    float *lev = sm + (warp * G + sub) * g.warp_floats;
-
-    const int Dout = (DOUT > 0) ? DOUT : a.Dout;
-    const int tpad = (DOUT > 0) ? pf_tpad_of(L) : a.tpad;
-    const int Wds = a.ndm_out / a.ndm_wt, Tds = a.nt_out / a.nt_wt;
-    // Weights of one subband for the warp's weight times tw0 .. tw0 + NT - 1, staged in shared memory
-    // as wsm[p * 32 + j] (lanes of one weight time read the same word, consecutive weight times
-    // consecutive words), and reloaded only when a multiplet's subband differs from the previous one.
-    const float *wrow = a.wt + ((long) b * a.ndm_wt + dm / Wds) * a.nt_wt * a.P * a.N;
-    const int tw0 = tout0 / Tds, NT = (Tds >= LW) ? 1 : LW / Tds;
-    const int tl = (lane < ntw) ? (tout / Tds - tw0) : 0;
-    float *wsm = lev + g.w_off;
-    int wsm_n = -1;
-    const Ts *pfrows = (const Ts *) a.pf + ((long) bt * a.ndm_out + dm) * a.M * a.pf_cap;
-    const int mask = int(a.pf_cap - 1);
-    // Window sample 0 (stream time s0 + 32 tile * Dout - tpad, a multiple of 4), as a delay-line slot.
-    long s0 = a.s0;
-    if constexpr (CTR) s0 = *a.chunk_ctr * (long) a.nt_chunk;
-    const int sbm = int((s0 + (long) tout0 * Dout - tpad) & (a.pf_cap - 1));
-    const bool full = (L > 1) || (a.P > 1);
-    const int nq0 = (ntw * Dout + tpad) >> 2;   // samples the active lanes read (a partial last tile reads fewer)
-
-    float best = -1.0e30f;
-    int winG = -1;            // group l * M + m of the first maximum; -1: no trial above -1e30
-    float outv = best;        // value and token of the first maximal trial
-    uint32_t tok = 0xffffffffu;
-    // Inputs of the winning group's first maximal pair, saved when the maximum moves, so that the
-    // token is found once at the end: x[j - 3S .. j] of its samples is = winP (a) and winP + 1 (b),
-    // the level's weights, and the pair's level, multiplet and start.
-    float xa0 = 0, xa1 = 0, xa2 = 0, xa3 = 0, xb0 = 0, xb1 = 0, xb2 = 0, xb3 = 0;
-    float sw0 = 0, sw1 = 0, sw2 = 0, sw3 = 0;
-    int winL = 0, winM = 0, winP = 0;
-
-    // The window's raw samples are staged with cp.async one multiplet ahead into alternating buffers
-    // (4-sample runs: a 4-aligned run never wraps the delay line). Level 0 is read from them.
-    Ts *raw0 = (Ts *) (lev + g.raw_off);
-    const int raw_ts = g.raw_floats * int(sizeof(float) / sizeof(Ts));
-    auto stage = [&](int m) {
-        const Ts *row = pfrows + (long) m * a.pf_cap;
-        Ts *raw = raw0 + (m & 1) * raw_ts;
-        for (int q = lane; q < nq0; q += LW)
-            cp_async_bytes<4 * sizeof(Ts)>(raw + 4 * q, row + ((sbm + 4 * q) & mask));
-        cp_async_commit();
-    };
-    stage(0);
-
-    for (int m = 0; m < a.M; m++) {
-        // Wait for this multiplet's samples; then stage the next one into the other buffer (every
-        // lane is past its reads of that buffer: they came before this loop's previous barriers).
-        cp_async_wait0();
-        __syncwarp();
-        if (m + 1 < a.M)
-            stage(m + 1);
-        const Ts *rawc = raw0 + (m & 1) * raw_ts;
-
-        const int n = a.m_to_n[m];
-        if (n != wsm_n) {
-            for (int idx = lane; idx < a.P * NT; idx += LW) {
-                const int p = idx / NT, j = idx - p * NT, t = tw0 + j;
-                wsm[p * 32 + j] = (t < a.nt_wt) ? wrow[((long) t * a.P + p) * a.N + n] : 0.0f;
-            }
-            __syncwarp();
-            wsm_n = n;
-        }
-#pragma unroll
-        for (int l = 0; l < L; l++) {
-            const int S = g.S[l], nsamp = g.nsamp[l];
-            const bool U = g.flags[l] & kPfU;
-            const bool nextU = (l + 1 < L) && (g.flags[l] & kPfNextU);
-
-            if (l > 0 && !U) {
-                // Saturated level (dt = Dcore): B_l[u] = B_{l-1}[rr u] + B_{l-1}[rr u + ss].
-                const int rr = g.rr[l], ss = g.ss[l];
-                for (int u = lane; u < g.n[l]; u += LW)
-                    lev[pf_phys(g, l, u)] = __fadd_rn(lev[pf_phys(g, l - 1, rr * u)], lev[pf_phys(g, l - 1, rr * u + ss)]);
-                __syncwarp();
-            }
-            if (nextU) {
-                // Entries of level l+1 before the first output time.
-                for (int u = lane; u < g.I[l + 1]; u += LW)
-                    lev[pf_phys(g, l + 1, u)] = (l == 0) ? __fadd_rn(to_f(rawc[2 * u]), to_f(rawc[2 * u + 1]))
-                                                        : __fadd_rn(lev[pf_phys(g, l, 2 * u)], lev[pf_phys(g, l, 2 * u + 1)]);
-            }
-
-            float w0 = 0.0f, w1 = 0.0f, w2 = 0.0f, w3 = 0.0f;
-            if (l == 0) w0 = wsm[tl];
-            if (full) {
-                w1 = wsm[(3 * l + 1) * 32 + tl];
-                w2 = wsm[(3 * l + 2) * 32 + tl];
-                w3 = wsm[(3 * l + 3) * 32 + tl];
-            }
-
-            const int j0 = g.I[l] + lane * nsamp;
-            float gmax = -1.0e30f;
-            int gp = 0;   // first fine sample (pair start) whose trials reach gmax
-            if (g.flags[l] & kPfPairs) {
-                // x0..x3 = x[is-3..is]; carried: x2, hx1 = x[is-2]/2, hx2 = x[is-1]/2, Ap = x[is-3]/2 + x[is-2].
-                // Level 0 comes from the raw staging buffer (entry i = raw sample i; j0 is a multiple of 4).
-                float x2, x1, x0;
-                if (l == 0) {
-                    float q[4];
-                    pf_load4<Ts>(rawc + j0 - 4, q);
-                    x0 = q[1]; x1 = q[2]; x2 = q[3];
-                } else {
-                    x2 = lev[pf_phys(g, l, j0 - 1)];
-                    x1 = lev[pf_phys(g, l, j0 - 2)];
-                    x0 = lev[pf_phys(g, l, j0 - 3)];
-                }
-                float2 H = make_float2(__fmul_rn(0.5f, x1), __fmul_rn(0.5f, x2));   // x[is-2]/2, x[is-1]/2
-                float Ap = __fadd_rn(__fmul_rn(0.5f, x0), x1);
-                const float *xs = lev + ((l > 0) ? pf_phys(g, l, j0) : 0);
-                float *ys = lev + (nextU ? pf_phys(g, l + 1, g.I[l + 1] + lane * (nsamp >> 1)) : 0);
-                const float2 W0 = make_float2(w0, w0), W1 = make_float2(w1, w1);
-                const float2 W2 = make_float2(w2, w2), W3 = make_float2(w3, w3);
-
-                // The trials of fine samples is (xa) and is + 1 (xb).
-                auto pair = [&](const float xa, const float xb, const int is) {
-                    const float2 X = make_float2(xa, xb);
-                    float mx;
-                    if (full) {
-                        // Fine samples is (xa) and is+1 (xb), in packed pairs (a, b): profiles
-                        // y1 = x2+x3, y2 = (x1/2+x2)+x3/2, y3 = ((x0/2+x1)+x2)+x3/2 with the reference's
-                        // association; A = x1/2+x2 of each sample, and y3's (x0/2+x1) is the previous A.
-                        const float2 Hn = f2mul(make_float2(0.5f, 0.5f), X);
-                        const float2 Pr = make_float2(x2, xa);       // x[is-1], x[is]
-                        const float2 A = f2add(H, Pr);
-                        const float2 V1 = f2mul(W1, f2add(Pr, X));
-                        const float2 V2 = f2mul(W2, f2add(A, Hn));
-                        const float2 V3 = f2mul(W3, f2add(f2add(make_float2(Ap, A.x), Pr), Hn));
-                        if (l == 0) {
-                            const float2 V0 = f2mul(W0, X);
-                            mx = fmaxf(pf_max3(V0.x, V1.x, V2.x), pf_max3(V3.x, V0.y, V1.y));
-                            mx = pf_max3(mx, V2.y, V3.y);
-                        } else {
-                            mx = fmaxf(pf_max3(V1.x, V2.x, V3.x), pf_max3(V1.y, V2.y, V3.y));
-                        }
-                        H = Hn; x2 = xb; Ap = A.y;
-                    } else {
-                        mx = fmaxf(__fmul_rn(w0, xa), __fmul_rn(w0, xb));
-                    }
-                    if (mx > gmax) { gmax = mx; gp = is; }
-                    if (nextU) ys[is >> 1] = __fadd_rn(xa, xb);
-                };
-                if (l == 0) {
-                    // 16-byte loads when runs of 8 stay 16-byte aligned (tpad and Dout multiples of 8)
-                    if (DOUT > 0 && nsamp % 8 == 0 && pf_tpad_of(L) % 8 == 0) {
-                        for (int is = 0; is < nsamp; is += 8) {
-                            float q[8];
-                            pf_load8<Ts>(rawc + j0 + is, q);
-                            pair(q[0], q[1], is);
-                            pair(q[2], q[3], is + 2);
-                            pair(q[4], q[5], is + 4);
-                            pair(q[6], q[7], is + 6);
-                        }
-                    } else {
-                        for (int is = 0; is < nsamp; is += 4) {
-                            float q[4];
-                            pf_load4<Ts>(rawc + j0 + is, q);
-                            pair(q[0], q[1], is);
-                            pair(q[2], q[3], is + 2);
-                        }
-                    }
-                } else {
-#pragma unroll 2
-                    for (int is = 0; is < nsamp; is += 2) {
-                        const float2 X = *(const float2 *) (xs + is);
-                        pair(X.x, X.y, is);
-                    }
-                }
-            } else {
-                // Levels stored without padding (contiguous across lanes): x[j - k S] = xb[is - k S].
-                const float *xb = lev + pf_phys(g, l, j0);
-                if (nsamp >= 2) {
-                    // Two fine samples at a time (S and nsamp even: 8-byte aligned pairs).
-                    for (int is = 0; is < nsamp; is += 2) {
-                        const float2 p3 = *(const float2 *) (xb + is), p2 = *(const float2 *) (xb + is - S);
-                        const float2 p1 = *(const float2 *) (xb + is - 2 * S), p0 = *(const float2 *) (xb + is - 3 * S);
-                        float mx;
-                        if (full) {
-                            const float ha = __fmul_rn(0.5f, p3.x), hb = __fmul_rn(0.5f, p3.y);
-                            const float v1a = __fmul_rn(w1, __fadd_rn(p2.x, p3.x));
-                            const float v2a = __fmul_rn(w2, __fadd_rn(__fadd_rn(__fmul_rn(0.5f, p1.x), p2.x), ha));
-                            const float v3a = __fmul_rn(w3, __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(0.5f, p0.x), p1.x), p2.x), ha));
-                            const float v1b = __fmul_rn(w1, __fadd_rn(p2.y, p3.y));
-                            const float v2b = __fmul_rn(w2, __fadd_rn(__fadd_rn(__fmul_rn(0.5f, p1.y), p2.y), hb));
-                            const float v3b = __fmul_rn(w3, __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(0.5f, p0.y), p1.y), p2.y), hb));
-                            mx = fmaxf(pf_max3(v1a, v2a, v3a), pf_max3(v1b, v2b, v3b));
-                            if (l == 0) mx = pf_max3(mx, __fmul_rn(w0, p3.x), __fmul_rn(w0, p3.y));
-                        } else {
-                            mx = fmaxf(__fmul_rn(w0, p3.x), __fmul_rn(w0, p3.y));
-                        }
-                        if (mx > gmax) { gmax = mx; gp = is; }
-                    }
-                } else {
-                    const float x3 = xb[0];
-                    float v = (l == 0) ? __fmul_rn(w0, x3) : -1.0e30f;
-                    if (full) {
-                        const float x0 = xb[-3 * S], x1 = xb[-2 * S], x2 = xb[-S];
-                        const float hx3 = __fmul_rn(0.5f, x3);
-                        const float y1 = __fadd_rn(x2, x3);
-                        const float y2 = __fadd_rn(__fadd_rn(__fmul_rn(0.5f, x1), x2), hx3);
-                        const float y3 = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(0.5f, x0), x1), x2), hx3);
-                        v = fmaxf(v, pf_max3(__fmul_rn(w1, y1), __fmul_rn(w2, y2), __fmul_rn(w3, y3)));
-                    }
-                    if (v > gmax) { gmax = v; gp = 0; }
-                }
-            }
-            __syncwarp();
-
-            const int G = l * a.M + m;
-            if (gmax > best || (gmax == best && G < winG)) {
-                best = gmax;
-                winG = G;
-                winL = l;
-                winM = m;
-                winP = gp;
-                const int S = g.S[l];
-                const int j = g.I[l] + lane * nsamp + gp;
-                // level l's entry i (level 0: the raw sample)
-                auto X = [&](int i) { return (l == 0) ? to_f(rawc[i]) : lev[pf_phys(g, l, i)]; };
-                xa3 = X(j);
-                if (full) {
-                    xa2 = X(j - S);
-                    xa1 = X(j - 2 * S);
-                    xa0 = X(j - 3 * S);
-                }
-                if (gp + 1 < nsamp) {
-                    xb3 = X(j + 1);
-                    if (full) {
-                        xb2 = X(j + 1 - S);
-                        xb1 = X(j + 1 - 2 * S);
-                        xb0 = X(j + 1 - 3 * S);
-                    }
-                }
-                sw0 = w0; sw1 = w1; sw2 = w2; sw3 = w3;
-            }
-        }
-
-    }
-
-    // The first trial of the winning pair, in the reference's order (fine time, then profile 0, 3l+1,
-    // 3l+2, 3l+3), equal to the maximum gives the output value and token.
-    if (winG >= 0) {
-        const int l = winL;
-        const uint32_t dt = uint32_t(gr.dt[l]);
-        const int nsamp = gr.nsamp[l];
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            if (k == 1 && winP + 1 >= nsamp) break;
-            const float x3 = k ? xb3 : xa3, x2 = k ? xb2 : xa2, x1 = k ? xb1 : xa1, x0 = k ? xb0 : xa0;
-            const uint32_t tk0 = (uint32_t(winM) << 16) | (uint32_t(winP + k) * dt);
-            if (l == 0) {
-                const float v0 = __fmul_rn(sw0, x3);
-                if (v0 == best) { outv = v0; tok = tk0; break; }
-            }
-            if (full) {
-                const float hx3 = __fmul_rn(0.5f, x3);
-                const float v1 = __fmul_rn(sw1, __fadd_rn(x2, x3));
-                const float v2 = __fmul_rn(sw2, __fadd_rn(__fadd_rn(__fmul_rn(0.5f, x1), x2), hx3));
-                const float v3 = __fmul_rn(sw3, __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(0.5f, x0), x1), x2), hx3));
-                if (v1 == best) { outv = v1; tok = tk0 | (uint32_t(3 * l + 1) << 8); break; }
-                if (v2 == best) { outv = v2; tok = tk0 | (uint32_t(3 * l + 2) << 8); break; }
-                if (v3 == best) { outv = v3; tok = tk0 | (uint32_t(3 * l + 3) << 8); break; }
-            }
-        }
-    }
-
-    if (!active)
-        return;
-    const long o = ((long) b * a.ndm_out + dm) * a.nt_out + tout;
-    ((Ts *) a.out_max)[o] = from_f<Ts>(outv);
-    a.out_argmax[o] = tok;
-}
-
-// DOUT > 0: compiled for that output time downsampling (with Dcore = min(DOUT, 8) and the plan's tpad
-// for L levels); DOUT = 0: any Dout >= 4, geometry read from the launch arguments.
-template<typename Ts, int L, int DOUT, bool CTR, int LW = 32>
-__global__ void __launch_bounds__(kPfWarps * 32) pf_fast_kernel(PfArgs a, PfGeom gr)
-{
-    if constexpr (DOUT > 0) {
-        constexpr PfGeom gc = pf_geom(DOUT, pf_dcore_of(DOUT), pf_tpad_of(L), L, sizeof(Ts), LW);
-        pf_fast_body<Ts, L, DOUT, CTR, LW>(a, gc, gr);
-    } else {
-        pf_fast_body<Ts, L, 0, CTR, LW>(a, gr, gr);
-    }
-}
-
-
-// -------------------------------------------------------------------------------------------------
 // Host launchers.
 
 
@@ -1415,56 +925,9 @@ int pf_warp_floats(int Dout, int tpad, int Dcore, int L)
 }
 
 
-// The fast kernel needs 4-sample runs of the window (Dout >= 4, tpad and s0 multiples of 4).
-static bool pf_fast_ok(const PfArgs &a)
-{
-    const long s0 = a.chunk_ctr ? (long) a.nt_chunk : a.s0;   // with a counter, s0 is a multiple of nt_chunk
-    return !a.force_general && a.Dout >= 4 && (a.tpad % 4) == 0 && (s0 % 4) == 0 && (a.pf_cap % 4) == 0 && a.L <= 5 && a.P <= kPfMaxProfiles;
-}
-
-template<typename Ts, int L, int DOUT, int LW = 32>
-static void launch_pf_fast(const PfArgs &a, const PfGeom &g, int B, cudaStream_t s)
-{
-    // g: the geometry for LW lanes per coarse DM
-    constexpr int G = 32 / LW;
-    size_t sm = (size_t) kPfWarps * G * g.warp_floats * sizeof(float);
-    dim3 grid((a.nt_out + LW - 1) / LW, (a.ndm_out + kPfWarps * G - 1) / (kPfWarps * G), B);
-    if (a.chunk_ctr) {
-        set_smem(pf_fast_kernel<Ts, L, DOUT, true, LW>, sm);
-        pf_fast_kernel<Ts, L, DOUT, true, LW><<<grid, kPfWarps * 32, sm, s>>>(a, g);
-    } else {
-        set_smem(pf_fast_kernel<Ts, L, DOUT, false, LW>, sm);
-        pf_fast_kernel<Ts, L, DOUT, false, LW><<<grid, kPfWarps * 32, sm, s>>>(a, g);
-    }
-    check_launch("pf_fast_kernel");
-}
-
 template<typename Ts, int L>
 static void launch_pf_l(const PfArgs &a, int B, cudaStream_t s)
 {
-    if (pf_fast_ok(a)) {
-        const PfGeom g = pf_geom(a.Dout, a.Dcore, a.tpad, L, (int) sizeof(Ts));
-        // Compiled geometries for the usual output downsamplings (pirate's default Dout = 2^pf_rank).
-        const bool std_geom = (a.Dcore == pf_dcore_of(a.Dout)) && (a.tpad == pf_tpad_of(L));
-        // Trees with 16 or 8 output times per chunk (the most downsampled primary trees) share a warp
-        // between 2 or 4 coarse DMs, so that no lane idles (compiled for the benchmark's Dout 16, widths
-        // to 32).
-        if constexpr (L == 5) {
-            if (std_geom && a.Dout == 16 && a.nt_out <= 8) {
-                launch_pf_fast<Ts, L, 16, 8>(a, pf_geom(a.Dout, a.Dcore, a.tpad, L, (int) sizeof(Ts), 8), B, s);
-                return;
-            }
-            if (std_geom && a.Dout == 16 && a.nt_out <= 16) {
-                launch_pf_fast<Ts, L, 16, 16>(a, pf_geom(a.Dout, a.Dcore, a.tpad, L, (int) sizeof(Ts), 16), B, s);
-                return;
-            }
-        }
-        if (std_geom && a.Dout == 16) launch_pf_fast<Ts, L, 16>(a, g, B, s);
-        else if (std_geom && a.Dout == 8) launch_pf_fast<Ts, L, 8>(a, g, B, s);
-        else if (std_geom && a.Dout == 4) launch_pf_fast<Ts, L, 4>(a, g, B, s);
-        else launch_pf_fast<Ts, L, 0>(a, g, B, s);
-        return;
-    }
     int wf = pf_warp_floats(a.Dout, a.tpad, a.Dcore, a.L);
     size_t sm = (size_t) kPfWarps * wf * sizeof(float);
     set_smem(pf_kernel<Ts, L>, sm);
@@ -1489,6 +952,15 @@ static void launch_pf_t(const PfArgs &a, int B, cudaStream_t s)
 void launch_pf(const PfArgs &a, int dtype, int B, cudaStream_t s)
 {
     if (a.Dout > 64 || a.Dout < 1) throw std::runtime_error("pf_kernel: time downsampling must be in [1, 64]");
+    // The register kernel wherever its geometry applies, that is for every plan with a time downsampling of 2 to 64
+    // (measured at 2 to 16: 1 beam of rank 10 15 -> 11 us, 8 beams of rank 16 1434 -> 922 us); the general one for a
+    // time downsampling of 1 or above 64.
+    if (pf_reg_ok(a)) {
+        if (dtype == 0) launch_pf_reg_f32(a, B, s);
+        else if (dtype == 1) launch_pf_reg_f16(a, B, s);
+        else launch_pf_reg_bf16(a, B, s);
+        return;
+    }
     if (dtype == 0) launch_pf_t<float>(a, B, s);
     else if (dtype == 1) launch_pf_t<__half>(a, B, s);
     else launch_pf_t<__nv_bfloat16>(a, B, s);

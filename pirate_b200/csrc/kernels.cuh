@@ -90,7 +90,7 @@ struct PfArgs
     int beam0;
     const long *chunk_ctr;  // if not null: s0 = *chunk_ctr * nt_chunk
     int nt_chunk;
-    int force_general;      // 1: the general kernel even where the fast one applies
+    int force_general;      // 1: the general kernel even where the register one applies
 };
 
 // Arguments of the fused tree-gridding + lagged-downsampling kernel.
@@ -198,6 +198,19 @@ void launch_stage1_halo_bf16(const Stage1Args &a, int nblocks, int B, cudaStream
 void launch_stage2_halo_f32(const Stage2Multi &m, bool sub, int nblocks, int B, cudaStream_t s);
 void launch_stage2_halo_f16(const Stage2Multi &m, bool sub, int nblocks, int B, cudaStream_t s);
 void launch_stage2_halo_bf16(const Stage2Multi &m, bool sub, int nblocks, int B, cudaStream_t s);
+
+// Whether pf_reg_kernel applies: the plan's geometry (Dcore = min(Dout, 8), tpad for L levels), Dout a power of two
+// from 2 to 64, rows at least a 16-byte chunk apart.
+inline bool pf_reg_ok(const PfArgs &a)
+{
+    const int tpad = (2 << a.L) > 4 ? (2 << a.L) : 4;
+    return !a.force_general && a.Dout >= 2 && a.Dout <= 64 && (a.Dout & (a.Dout - 1)) == 0 && a.Dcore == (a.Dout < 8 ? a.Dout : 8) &&
+           a.tpad == tpad && a.L >= 1 && a.L <= 5 && (a.P == 3 * a.L + 1 || (a.L == 1 && a.P == 1)) && a.pf_cap >= 64;
+}
+// One translation unit per storage type (pf_reg_*.cu).
+void launch_pf_reg_f32(const PfArgs &a, int B, cudaStream_t s);
+void launch_pf_reg_f16(const PfArgs &a, int B, cudaStream_t s);
+void launch_pf_reg_bf16(const PfArgs &a, int B, cudaStream_t s);
 void launch_pf(const PfArgs &a, int dtype, int B, cudaStream_t s);
 
 struct DedispersionPlan;
