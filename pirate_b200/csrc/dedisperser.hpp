@@ -49,7 +49,7 @@ struct GroupTuning
 {
     bool merge_stage2 = true;   // one stage-2 grid for consecutive trees with the same kernel
     bool pf_general = false;    // the general peak-finding kernel even where the fast one applies
-    int grid_block = 128;       // threads per gridding block (a multiple of the windows per row; <= 512)
+    int grid_block = 128;       // threads per block of grid_lds_kernel (a multiple of the windows per row; <= 512)
 };
 
 class GpuDedisperser

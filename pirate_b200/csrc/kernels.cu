@@ -1,6 +1,6 @@
 // kernels.cu -- sm_100a kernels of the B200 dedispersion path.
 //
-//   grid_lds_kernel  tree gridding + lagged downsampling (replaces GpuTreeGriddingKernel,
+//   grid_warp_kernel, grid_lds_kernel  tree gridding + lagged downsampling (replace GpuTreeGriddingKernel,
 //                    src_lib/TreeGriddingKernel.cu:108-279, and GpuLaggedDownsamplingKernel,
 //                    src_lib/GpuLaggedDownsamplingKernel.cu:668-918)
 //   pf_kernel      peak finding, max/argmax      (replaces the pf half of CoalescedDdKernel2 / GpuPeakFindingKernel)
@@ -34,8 +34,8 @@ namespace pb2 {
 // 2^s1dd - 1 - (c mod 2^s1dd) (ReferenceLaggedDownsamplingKernel.cpp:46-57), so that the stage-1
 // kernel reads aligned rows.
 //
-// One thread per (beam, tree-channel pair (2c, 2c+1), window of W0 level-0 samples); consecutive
-// threads take consecutive windows, so every load and store is a contiguous run across the warp.
+// grid_lds_kernel, for chunk lengths or level counts that grid_warp_kernel below does not take: one thread per (beam,
+// tree-channel pair (2c, 2c+1), window of W0 level-0 samples); consecutive threads take consecutive windows, so every load and store is a contiguous run across the warp.
 // The thread grids both channels of its window (and writes them as the level-0 tree), builds every
 // level in registers, and gets the even channel's predecessor sample at each level by gridding the
 // 2^nlev samples before its window (at the chunk start: from a parity double-buffered state).
@@ -134,65 +134,6 @@ __device__ __forceinline__ void grid_run(const GridLdsArgs &a, int b, long n, lo
             load_run<Ts, W>((const Ts *) a.in + row * a.T + t0, x);
 #pragma unroll
         for (int i = 0; i < W; i++) o[i] = __fadd_rn(o[i], __fmul_rn(w, x[i]));
-    }
-}
-
-// int4 gridding through per-warp lookup tables. A warp's 32 windows of one tree-channel pair read the
-// same few input rows, each input sample once per tree channel that overlaps its row (about 2.5 times
-// at rank 16 from 16384 channels). Instead of dequantizing on every read, the warp first tabulates,
-// per (row, 256-sample scale block), the 16 values its nibbles can take, rounded to Ts exactly as
-// load_run_q rounds them; each read is then a nibble extract and a shared-memory lookup.
-constexpr int kLutRows = 8;   // input rows per channel pair served by the tables
-
-// Table of the warp: lut[(r * NBLK + blk) * 16 + u] = sample value of nibble u in row rlo + r, scale
-// block blk0 + blk.
-template<typename Ts, int NBLK>
-__device__ __forceinline__ void lut_build(const GridLdsArgs &a, int b, int rlo, int nrows, long blk0, float *lut, int lane)
-{
-    const __half2 *so = (const __half2 *) a.q_scoff;
-    const long nsb = a.T >> 8;
-    for (int e = lane; e < nrows * NBLK * 16; e += 32) {
-        const int r = e / (NBLK * 16), blk = (e / 16) % NBLK, u = e & 15;
-        const float2 sc = __half22float2(so[((long) b * a.F + rlo + r) * nsb + blk0 + blk]);
-        lut[e] = to_f(from_f<Ts>(dq_value(uint32_t(u), sc.x, sc.y)));
-    }
-    __syncwarp();
-}
-
-// The nibble words of a window of W samples (W / 8 words) of input row 'row' (t0 a multiple of 8).
-template<int W>
-__device__ __forceinline__ void lut_words(const GridLdsArgs &a, long row, long t0, uint32_t (&q)[W / 8])
-{
-    const uint32_t *p = (const uint32_t *) ((const uint8_t *) a.q_data + row * (a.T >> 1) + (t0 >> 1));
-#pragma unroll
-    for (int v = 0; v < W / 8; v++) q[v] = p[v];
-}
-
-// o += w * (row's samples), the samples looked up in table L.
-template<int W>
-__device__ __forceinline__ void lut_accum(float (&o)[W], float w, const uint32_t (&q)[W / 8], const float *L)
-{
-#pragma unroll
-    for (int v = 0; v < W / 8; v++)
-#pragma unroll
-        for (int k8 = 0; k8 < 8; k8++) o[8 * v + k8] = __fadd_rn(o[8 * v + k8], __fmul_rn(w, L[(q[v] >> (4 * k8)) & 15]));
-}
-
-// grid_run<Ts, W, true> of tree channel n through the warp's tables (W a multiple of 8, t0 in scale
-// block blk0 + myblk), summed in ascending input channel. q0 holds the words of the channel's first
-// input row (loaded by the caller before the tables were built); later rows are loaded here.
-template<typename Ts, int W, int NBLK>
-__device__ __forceinline__ void grid_run_lut(const GridLdsArgs &a, int b, int f0, int cnt, int woff, long t0, float (&o)[W],
-                                             const uint32_t (&q0)[W / 8], const float *lut, int rlo, int myblk)
-{
-#pragma unroll
-    for (int i = 0; i < W; i++) o[i] = 0.0f;
-    if (cnt > 0)
-        lut_accum<W>(o, a.chan_w[woff], q0, lut + ((f0 - rlo) * NBLK + myblk) * 16);
-    for (int k = 1; k < cnt; k++) {
-        uint32_t q[W / 8];
-        lut_words<W>(a, (long) b * a.F + f0 + k, t0, q);
-        lut_accum<W>(o, a.chan_w[woff + k], q, lut + ((f0 + k - rlo) * NBLK + myblk) * 16);
     }
 }
 
@@ -536,10 +477,6 @@ __global__ void __launch_bounds__(kGridMaxThreads) grid_lds_kernel(GridLdsArgs a
     constexpr int W0 = ((1 << NLEV) > 8) ? (1 << NLEV) : 8;
     constexpr int WE = 1 << NLEV;           // level-0 samples feeding one level-NLEV sample
     __shared__ float xch[(NLEV > 0) ? NLEV : 1][kGridMaxThreads];
-    // int4 lookup tables (grid_run_lut): for windows of at most 16 samples, NBLK scale blocks per warp.
-    constexpr bool LUT = Q && (W0 <= 16);
-    constexpr int NBLK = LUT ? (32 * W0) / 256 : 1;
-    __shared__ float lut_sh[LUT ? (kGridMaxThreads / 32) * kLutRows * NBLK * 16 : 1];
 
     const long nhalf = 1L << (a.rank - 1);
     const long nwin = a.T / W0;
@@ -556,37 +493,9 @@ __global__ void __launch_bounds__(kGridMaxThreads) grid_lds_kernel(GridLdsArgs a
     const long t0 = (long) win * W0;
 
     float r0[W0], r1[W0];
-    // A warp uses the tables when its 32 threads are live windows of one channel pair (nwin a multiple
-    // of 32; blocks start at window 0) whose input rows fit; the choice is uniform across the warp.
-    bool use_lut = false;
-    if constexpr (LUT) {
-        if (live && (nwin & 31) == 0) {
-            const int fa = a.chan_f0[2 * c], ca = a.chan_cnt[2 * c], fb = a.chan_f0[2 * c + 1], cb = a.chan_cnt[2 * c + 1];
-            const int rlo = min(ca ? fa : fb, cb ? fb : fa);
-            const int rhi = max(fa + ca, fb + cb);
-            use_lut = (rhi - rlo) <= kLutRows;
-            if (use_lut) {
-                // The first input row of each channel is loaded before the tables are built, so that its
-                // latency overlaps that of the (scale, offset) loads.
-                uint32_t qa[W0 / 8], qb[W0 / 8];
-                lut_words<W0>(a, (long) b * a.F + (ca ? fa : rlo), t0, qa);
-                lut_words<W0>(a, (long) b * a.F + (cb ? fb : rlo), t0, qb);
-                const int wa = a.chan_woff[2 * c], wb = a.chan_woff[2 * c + 1];
-                const int lane = threadIdx.x & 31;
-                const long blk0 = ((long) (win - lane) * W0) >> 8;
-                float *lut = lut_sh + (threadIdx.x >> 5) * (kLutRows * NBLK * 16);
-                lut_build<Ts, NBLK>(a, b, rlo, rhi - rlo, blk0, lut, lane);
-                const int myblk = int((t0 >> 8) - blk0);
-                grid_run_lut<Ts, W0, NBLK>(a, b, fa, ca, wa, t0, r0, qa, lut, rlo, myblk);
-                grid_run_lut<Ts, W0, NBLK>(a, b, fb, cb, wb, t0, r1, qb, lut, rlo, myblk);
-            }
-        }
-    }
-    if (live && !use_lut) {
+    if (live) {
         grid_run<Ts, W0, Q>(a, b, 2 * c, t0, r0);
         grid_run<Ts, W0, Q>(a, b, 2 * c + 1, t0, r1);
-    }
-    if (live) {
         Ts *lev0 = (Ts *) a.tree0 + ((long) b * (2 * nhalf) + 2 * c) * a.T + t0;
         store_run<Ts, W0>(lev0, r0);
         store_run<Ts, W0>(lev0 + a.T, r1);
@@ -661,6 +570,367 @@ __global__ void __launch_bounds__(kGridMaxThreads) grid_lds_kernel(GridLdsArgs a
     }
 }
 
+// ---------------------------------------------------------------------------------------------
+// The same by one warp per (beam, tree-channel pair): it goes through the chunk in steps of 32 windows of W samples, a
+// lane owning one window. The sample before a window comes from the lane before, and before a step from the step
+// before, so that nothing is exchanged between warps; the outputs leave in contiguous runs, through the warp's own
+// shared memory (written by each lane for its window, a level row's samples would be 2-byte stores 4 to 16 bytes
+// apart). The two channels of the pair are the halves of packed fp32 operations.
+//
+// int4 input goes through tables: an input sample is read by about 2.5 pairs at rank 16 from 16384 channels, so
+// per step the warp tabulates, for each input row of the pair and 256-sample scale block, the 16 values that a nibble
+// can take, rounded to the storage type; a sample is then a nibble extract and a shared-memory lookup.
+//
+// What bounds it: instruction issue (two thirds of the slots; 770 warp instructions per pair and 512-sample step with
+// int4 input and four levels) and the loads' latency at 20 to 32 warps per SM; the launch bounds are the fastest of those
+// tried. Against a thread per window (grid_lds_kernel, with 64-bit divisions to find its window, a block barrier and level
+// rows stored 2 bytes at a time), per chunk on a B200: 4 beams of rank 16, int4 to fp16, four levels 661 -> 480 us; 1 beam
+// of rank 16, fp32, four levels 313 -> 200 us; 2 beams of rank 16, fp16, no level 297 -> 128 us; 16 beams of rank 12, fp16,
+// two levels 215 -> 129 us. Staging the rows of 8 pairs in shared memory, each input sample read and dequantized once,
+// took 912, 264, 146 and 141 us: the pairs share too few rows to pay for the barriers.
+
+constexpr int kGridWarps = 4;   // warps per block: consecutive pairs, which share input rows
+constexpr int kLutRows = 8;     // input rows of a pair served by the tables
+
+// Packed fp32 pairs: each element is rounded to nearest like the scalar operation.
+__device__ __forceinline__ unsigned long long f2bits(float2 a)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+    return r;
+}
+__device__ __forceinline__ float2 f2from(unsigned long long r)
+{
+    float2 d;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(r));
+    return d;
+}
+__device__ __forceinline__ float2 f2bfly(float2 a, float2 b)
+{
+    unsigned long long s, d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(s) : "l"(f2bits(a)), "l"(f2bits(b)));
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(s), "l"(f2bits(make_float2(kRsqrt2, kRsqrt2))));
+    return f2from(d);
+}
+__device__ __forceinline__ float2 f2fma(float2 a, float2 b, float2 c)
+{
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(f2bits(a)), "l"(f2bits(b)), "l"(f2bits(c)));
+    return f2from(d);
+}
+
+// Two samples as one word of a 16-bit type.
+template<typename Ts>
+__device__ __forceinline__ uint32_t pack2(float x, float y)
+{
+    if constexpr (std::is_same<Ts, __half>::value) {
+        const __half2 h = __floats2half2_rn(x, y);
+        return *(const uint32_t *) &h;
+    } else {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+        return *(const uint32_t *) &h;
+    }
+}
+
+// N samples (a power of two) to p, in stores of up to 16 bytes.
+template<typename Ts, int N>
+__device__ __forceinline__ void store_vec(Ts *p, const float (&o)[N])
+{
+    if constexpr (sizeof(Ts) == 4) {
+        if constexpr (N >= 4) {
+#pragma unroll
+            for (int i = 0; i < N; i += 4) *(float4 *) (p + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+        } else if constexpr (N == 2) {
+            *(float2 *) p = make_float2(o[0], o[1]);
+        } else {
+            *p = o[0];
+        }
+    } else {
+        if constexpr (N >= 8) {
+#pragma unroll
+            for (int i = 0; i < N; i += 8)
+                *(uint4 *) (p + i) = make_uint4(pack2<Ts>(o[i], o[i + 1]), pack2<Ts>(o[i + 2], o[i + 3]), pack2<Ts>(o[i + 4], o[i + 5]),
+                                                pack2<Ts>(o[i + 6], o[i + 7]));
+        } else if constexpr (N == 4) {
+            *(uint2 *) p = make_uint2(pack2<Ts>(o[0], o[1]), pack2<Ts>(o[2], o[3]));
+        } else if constexpr (N == 2) {
+            *(uint32_t *) p = pack2<Ts>(o[0], o[1]);
+        } else {
+            *p = from_f<Ts>(o[0]);
+        }
+    }
+}
+
+template<typename Ts, int NLEV, int W, bool Q>
+struct GridWarp
+{
+    static constexpr int STEP = 32 * W;
+    static constexpr int NBLK = STEP / 256;                                   // scale blocks per step
+    static constexpr int LUT = Q ? kLutRows * NBLK * 16 * int(sizeof(float)) : 0;
+    static constexpr int OUT = STEP * int(sizeof(Ts));
+    static constexpr int BYTES = LUT > OUT ? LUT : OUT;                       // shared memory: the tables, then the outputs
+    // First sample of level p's row in the output buffer.
+    __host__ __device__ static constexpr int off(int p) { return STEP - (STEP >> (p - 1)); }
+};
+
+// The warp's 32 windows of W samples to p and on, through buf: 16-byte chunk c lies at c ^ (c / 8 mod CH), which leaves
+// neither side bank conflicts.
+template<typename Ts, int W>
+__device__ __forceinline__ void store_warp(Ts *p, const float (&o)[W], unsigned char *buf, int lane)
+{
+    constexpr int PER = 16 / sizeof(Ts), CH = W / PER;
+    if constexpr (CH == 1) {
+        store_vec<Ts, W>(p + lane * W, o);
+    } else {
+        auto at = [&](int c) { return (uint4 *) buf + (c ^ ((c >> 3) & (CH - 1))); };
+#pragma unroll
+        for (int v = 0; v < CH; v++) {
+            float x[PER];
+#pragma unroll
+            for (int i = 0; i < PER; i++) x[i] = o[v * PER + i];
+            store_vec<Ts, PER>((Ts *) at(lane * CH + v), x);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int v = 0; v < CH; v++) ((uint4 *) p)[v * 32 + lane] = *at(v * 32 + lane);
+        __syncwarp();
+    }
+}
+
+// The warp's N samples lev[0..N) (N a multiple of 16) to delay-line positions pos and on. 16-bit types move as words,
+// across the halves of two words where the first position is odd.
+template<typename Ts, int N>
+__device__ __forceinline__ void store_line(Ts *ring, int pos, int mask, const Ts *lev, int lane)
+{
+    if constexpr (sizeof(Ts) == 4) {
+#pragma unroll
+        for (int i0 = 0; i0 < N; i0 += 32) {
+            const int i = i0 + lane;
+            if (N % 32 == 0 || i < N) ring[(pos + i) & mask] = lev[i];
+        }
+    } else {
+        const uint32_t *w = (const uint32_t *) lev + lane;
+        uint32_t *o = (uint32_t *) ring;
+        const int p2 = (pos >> 1) + lane, m2 = mask >> 1;
+        if (pos & 1) {
+#pragma unroll
+            for (int j0 = 0; j0 < N / 2; j0 += 32)
+                if ((j0 > 0 || lane > 0) && (j0 + 32 <= N / 2 || j0 + lane < N / 2)) o[(p2 + j0) & m2] = __byte_perm(w[j0 - 1], w[j0], 0x5432);
+            if (lane < 2) ring[(pos + lane * (N - 1)) & mask] = lev[lane * (N - 1)];
+        } else {
+#pragma unroll
+            for (int j0 = 0; j0 < N / 2; j0 += 32)
+                if (j0 + 32 <= N / 2 || j0 + lane < N / 2) o[(p2 + j0) & m2] = w[j0];
+        }
+    }
+}
+
+// Levels p .. NLEV of a window, in place as in grid_lds_kernel, into the warp's rows. carry: the even channel's last
+// sample of every level before the step.
+template<typename Ts, int NLEV, int p, int W>
+__device__ __forceinline__ void warp_levels(float2 (&r)[W], float (&carry)[NLEV], Ts *lev, int lane)
+{
+    constexpr int len = W >> p;
+    float o[len];
+#pragma unroll
+    for (int u = 0; u < len; u++) r[u] = f2bfly(r[2 * u], r[2 * u + 1]);
+    const float up = __shfl_up_sync(0xffffffffu, r[len - 1].x, 1);
+    o[0] = bfly(lane == 0 ? carry[p - 1] : up, r[0].y);
+    carry[p - 1] = __shfl_sync(0xffffffffu, r[len - 1].x, 31);
+#pragma unroll
+    for (int u = 1; u < len; u++) o[u] = bfly(r[u - 1].x, r[u].y);
+    store_vec<Ts, len>(lev + GridWarp<Ts, NLEV, W, false>::off(p) + lane * len, o);
+    if constexpr (p < NLEV) warp_levels<Ts, NLEV, p + 1, W>(r, carry, lev, lane);
+}
+
+template<typename Ts, int NLEV, int p, int W>
+__device__ __forceinline__ void warp_lines(const GridLdsArgs &a, long row, unsigned u, unsigned lag, const Ts *lev, int lane)
+{
+    // row: the pair's row of the delay lines; u: the step's first level-0 sample (its low bits)
+    using G = GridWarp<Ts, NLEV, W, false>;
+    const int mask = int(a.cap_mask[p - 1]);
+    store_line<Ts, (G::STEP >> p)>((Ts *) a.ring[p - 1] + row * (mask + 1), int((u >> p) + lag) & mask, mask, lev + G::off(p), lane);
+    if constexpr (p < NLEV) warp_lines<Ts, NLEV, p + 1, W>(a, row, u, lag, lev, lane);
+}
+
+// Sample k8 of a nibble word, from the table at shared address L (a multiple of 64).
+__device__ __forceinline__ float lut_at(uint32_t L, uint32_t q, int k8)
+{
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(L | ((k8 ? q >> (4 * k8 - 2) : q << 2) & 0x3cu)));
+    return v;
+}
+
+// The nibble words of W samples at p.
+template<int W>
+__device__ __forceinline__ void lut_words(const unsigned char *p, uint32_t (&q)[W / 8])
+{
+    if constexpr (W == 16) {
+        const uint2 w = *(const uint2 *) p;
+        q[0] = w.x;
+        q[1] = w.y;
+    } else {
+        q[0] = *(const uint32_t *) p;
+    }
+}
+
+template<typename Ts, int NLEV, int W, bool Q>
+__global__ void __launch_bounds__(32 * kGridWarps, W == 16 ? (Q ? 6 : 5) : 8) grid_warp_kernel(GridLdsArgs a)
+{
+    using G = GridWarp<Ts, NLEV, W, Q>;
+    constexpr int STEP = G::STEP;
+    __shared__ __align__(128) unsigned char grid_sm[kGridWarps * G::BYTES];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned char *wsm = grid_sm + warp * G::BYTES;
+    const int nhalf = 1 << (a.rank - 1);
+    const int c = blockIdx.x * kGridWarps + warp, b = blockIdx.y, bt = a.beam0 + b;
+    if (c >= nhalf) return;   // whole warps; nothing below waits for another warp
+    const long ichunk = a.chunk_ctr ? *a.chunk_ctr : a.ichunk;
+    const int parity = int(ichunk & 1);
+    // This warp's steps: a share of the chunk's where pairs alone are too few for the GPU.
+    const int nsteps = a.T / STEP;
+    const int s0 = nsteps * int(blockIdx.z) / int(gridDim.z), s1 = nsteps * (int(blockIdx.z) + 1) / int(gridDim.z);
+
+    const int fa = a.chan_f0[2 * c], ca = a.chan_cnt[2 * c], fb = a.chan_f0[2 * c + 1], cb = a.chan_cnt[2 * c + 1];
+    const float *wa = a.chan_w + a.chan_woff[2 * c], *wb = a.chan_w + a.chan_woff[2 * c + 1];
+    const float2 w0 = make_float2(ca > 0 ? wa[0] : 0.0f, cb > 0 ? wb[0] : 0.0f);
+    Ts *tree = (Ts *) a.tree0 + ((long) b * (2 * nhalf) + 2 * c) * a.T;
+
+    float carry[NLEV > 0 ? NLEV : 1];
+    const unsigned u0 = unsigned(ichunk * a.T);   // low bits of the chunk's first sample: delay lines have fewer than 2^27 slots
+    const unsigned lag = (1u << a.lag_rank) - 1 - (c & ((1u << a.lag_rank) - 1));
+    if constexpr (NLEV > 0) {
+        if (s0 == 0) {
+#pragma unroll
+            for (int p = 1; p <= NLEV; p++)
+                carry[p - 1] = a.state[(((long) parity * a.total_beams + bt) * a.nlev + (p - 1)) * nhalf + c];
+        } else {
+            // the even channel's 2^NLEV samples before, one per lane
+            constexpr int WE = 1 << NLEV;
+            float e[1];
+            grid_run<Ts, 1, Q>(a, b, 2 * c, (long) s0 * STEP - WE + (lane & (WE - 1)), e);
+#pragma unroll
+            for (int p = 1; p <= NLEV; p++) {
+                e[0] = bfly(e[0], __shfl_xor_sync(0xffffffffu, e[0], 1 << (p - 1)));
+                carry[p - 1] = __shfl_sync(0xffffffffu, e[0], WE - 1);
+            }
+        }
+    }
+
+    // int4: the pair's input rows from rlo on, if they fit the tables, and the step's words of the first ones.
+    const int rlo = min(ca ? fa : fb, cb ? fb : fa), rows = max(fa + ca, fb + cb) - rlo;
+    const bool use_lut = Q && rows <= kLutRows;
+    const unsigned char *qa = nullptr, *qb = nullptr;
+    const __half2 *so = nullptr;
+    uint32_t la = 0, lb = 0, va[W / 8], vb[W / 8];
+    float fv = 0.0f;
+    if constexpr (Q) {
+        const unsigned char *q = (const unsigned char *) a.q_data + (long) b * a.F * (a.T >> 1) + (s0 * STEP + lane * W) / 2;
+        qa = q + (long) (ca ? fa : rlo) * (a.T >> 1);
+        qb = q + (long) (cb ? fb : rlo) * (a.T >> 1);
+        so = (const __half2 *) a.q_scoff + ((long) b * a.F + rlo) * (a.T >> 8) + ((s0 * STEP) >> 8) + (G::NBLK == 2 ? lane >> 4 : 0);
+        const uint32_t L = (uint32_t) __cvta_generic_to_shared(wsm) + (G::NBLK == 2 ? (lane >> 4) * 64 : 0);
+        la = L + (ca ? fa - rlo : 0) * G::NBLK * 64;
+        lb = L + (cb ? fb - rlo : 0) * G::NBLK * 64;
+        fv = float(((lane & 15) ^ 8) - 8);   // the nibble this lane tabulates
+        if (use_lut) {
+            lut_words<W>(qa, va);
+            lut_words<W>(qb, vb);
+        }
+    }
+
+    for (int s = s0; s < s1; s++) {
+        const int t0 = s * STEP + lane * W;
+        float2 r[W];   // the channels' samples: even (x) and odd (y)
+        if (use_lut) {
+#pragma unroll 1
+            for (int k = 0; k < rows; k++) {
+                const float2 sc = __half22float2(so[(long) k * (a.T >> 8)]);
+                const float x = (lane & 15) == 8 ? 0.0f : to_f(from_f<Ts>(__fadd_rn(__fmul_rn(sc.x, fv), sc.y)));
+                if (G::NBLK == 2 || lane < 16) ((float *) wsm)[k * G::NBLK * 16 + lane] = x;
+            }
+            so += G::NBLK;
+            __syncwarp();
+            // The first row's products are added to zero by one fused multiply-add, which rounds like the product.
+#pragma unroll
+            for (int i = 0; i < W; i++)
+                r[i] = f2fma(w0, make_float2(lut_at(la, va[i / 8], i & 7), lut_at(lb, vb[i / 8], i & 7)), make_float2(0.0f, 0.0f));
+            if (ca == 0 || cb == 0)   // a channel without input is zero, whatever the tables hold
+#pragma unroll
+                for (int i = 0; i < W; i++) r[i] = make_float2(ca ? r[i].x : 0.0f, cb ? r[i].y : 0.0f);
+#pragma unroll 1
+            for (int k = 1; k < ca; k++) {
+                lut_words<W>(qa + (long) k * (a.T >> 1), va);
+                const float wk = wa[k];
+#pragma unroll
+                for (int i = 0; i < W; i++) r[i].x = __fadd_rn(r[i].x, __fmul_rn(wk, lut_at(la + k * G::NBLK * 64, va[i / 8], i & 7)));
+            }
+#pragma unroll 1
+            for (int k = 1; k < cb; k++) {
+                lut_words<W>(qb + (long) k * (a.T >> 1), vb);
+                const float wk = wb[k];
+#pragma unroll
+                for (int i = 0; i < W; i++) r[i].y = __fadd_rn(r[i].y, __fmul_rn(wk, lut_at(lb + k * G::NBLK * 64, vb[i / 8], i & 7)));
+            }
+            qa += STEP / 2;
+            qb += STEP / 2;
+            if (s + 1 < s1) {
+                lut_words<W>(qa, va);
+                lut_words<W>(qb, vb);
+            }
+            __syncwarp();   // the tables' memory is the outputs' from here on
+        } else if constexpr (Q) {
+            float x[W];
+            grid_run<Ts, W, Q>(a, b, 2 * c, t0, x);
+#pragma unroll
+            for (int i = 0; i < W; i++) r[i].x = x[i];
+            grid_run<Ts, W, Q>(a, b, 2 * c + 1, t0, x);
+#pragma unroll
+            for (int i = 0; i < W; i++) r[i].y = x[i];
+        } else {
+            const Ts *in = (const Ts *) a.in + (long) b * a.F * a.T + t0;
+            float x[W], y[W];
+#pragma unroll
+            for (int i = 0; i < W; i++) x[i] = y[i] = 0.0f;
+            if (ca > 0) load_run<Ts, W>(in + (long) fa * a.T, x);
+            if (cb > 0) load_run<Ts, W>(in + (long) fb * a.T, y);
+#pragma unroll
+            for (int i = 0; i < W; i++) r[i] = f2fma(w0, make_float2(x[i], y[i]), make_float2(0.0f, 0.0f));
+#pragma unroll 1
+            for (int k = 1; k < ca; k++) {
+                load_run<Ts, W>(in + (long) (fa + k) * a.T, x);
+                const float wk = wa[k];
+#pragma unroll
+                for (int i = 0; i < W; i++) r[i].x = __fadd_rn(r[i].x, __fmul_rn(wk, x[i]));
+            }
+#pragma unroll 1
+            for (int k = 1; k < cb; k++) {
+                load_run<Ts, W>(in + (long) (fb + k) * a.T, y);
+                const float wk = wb[k];
+#pragma unroll
+                for (int i = 0; i < W; i++) r[i].y = __fadd_rn(r[i].y, __fmul_rn(wk, y[i]));
+            }
+        }
+        float x[W];
+#pragma unroll
+        for (int i = 0; i < W; i++) x[i] = r[i].x;
+        store_warp<Ts, W>(tree + s * STEP, x, wsm, lane);
+#pragma unroll
+        for (int i = 0; i < W; i++) x[i] = r[i].y;
+        store_warp<Ts, W>(tree + a.T + s * STEP, x, wsm, lane);
+        if constexpr (NLEV > 0) {
+            warp_levels<Ts, NLEV, 1, W>(r, carry, (Ts *) wsm, lane);
+            __syncwarp();
+            warp_lines<Ts, NLEV, 1, W>(a, (long) bt * nhalf + c, u0 + unsigned(s * STEP), lag, (const Ts *) wsm, lane);
+            __syncwarp();
+        }
+    }
+    if (NLEV > 0 && lane == 0 && s1 == nsteps) {
+#pragma unroll
+        for (int p = 1; p <= NLEV; p++)
+            a.state[(((long) (1 - parity) * a.total_beams + bt) * a.nlev + (p - 1)) * nhalf + c] = carry[p - 1];
+    }
+}
 
 // -------------------------------------------------------------------------------------------------
 // Peak finding. One warp per (beam, coarse dm, 32 consecutive output times). For each multiplet m
@@ -824,9 +1094,37 @@ __global__ void __launch_bounds__(kPfWarps * 32) pf_kernel(PfArgs a, int warp_fl
 // Host launchers.
 
 
+template<typename Ts, int NLEV, int W, bool Q>
+static void launch_grid_warp(const GridLdsArgs &a, cudaStream_t s)
+{
+    const int nblk = ((1 << (a.rank - 1)) + kGridWarps - 1) / kGridWarps, nsteps = a.T / (32 * W);
+    // Few pairs: split the chunk over up to 8 blocks per SM.
+    const int nz = std::max(1, std::min(nsteps, 8 * 148 / std::max(1, nblk * a.B)));
+    grid_warp_kernel<Ts, NLEV, W, Q><<<dim3(nblk, a.B, nz), 32 * kGridWarps, 0, s>>>(a);
+    check_launch("grid_warp_kernel");
+}
+
 template<typename Ts, int NLEV>
 static void launch_grid_lds_t(const GridLdsArgs &a, cudaStream_t s)
 {
+    if (a.q_data && a.T % 256) throw std::runtime_error("grid_lds_kernel: int4 input needs a chunk length that is a multiple of 256");
+    if constexpr (NLEV <= 4) {
+        // A warp per pair for whole steps, faster than a thread per window at every size measured (1 beam of rank 10
+        // 11 -> 10 us, of rank 8 the same; larger ones above grid_warp_kernel). 16-sample windows where the levels need
+        // them, and for int4 input, whose tables then have two scale blocks per step for the warp to fill.
+        if (a.T % 512 == 0 && (a.q_data || NLEV == 4)) {
+            if (a.q_data) launch_grid_warp<Ts, NLEV, 16, true>(a, s);
+            else if constexpr (NLEV == 4) launch_grid_warp<Ts, NLEV, 16, false>(a, s);
+            return;
+        }
+        if constexpr (NLEV < 4) {
+            if (a.T % 256 == 0) {
+                if (a.q_data) launch_grid_warp<Ts, NLEV, 8, true>(a, s);
+                else launch_grid_warp<Ts, NLEV, 8, false>(a, s);
+                return;
+            }
+        }
+    }
     constexpr int W0 = ((1 << NLEV) > 8) ? (1 << NLEV) : 8;
     if (a.T % W0) throw std::runtime_error("grid_lds_kernel: chunk length not a multiple of the window");
     const long nwin = a.T / W0;
@@ -836,7 +1134,6 @@ static void launch_grid_lds_t(const GridLdsArgs &a, cudaStream_t s)
     const int target = (a.block_target > 0) ? std::min(a.block_target, kGridMaxThreads) : 128;
     int bd = (nwin <= target) ? int(nwin * (target / nwin)) : (nwin <= kGridMaxThreads ? int(nwin) : kGridMaxThreads);
     if (a.q_data) {
-        if (a.T % 256) throw std::runtime_error("grid_lds_kernel: int4 input needs a chunk length that is a multiple of 256");
         grid_lds_kernel<Ts, NLEV, true><<<(unsigned) ((nthr + bd - 1) / bd), bd, 0, s>>>(a);
     } else {
         grid_lds_kernel<Ts, NLEV, false><<<(unsigned) ((nthr + bd - 1) / bd), bd, 0, s>>>(a);
@@ -953,7 +1250,7 @@ void launch_pf(const PfArgs &a, int dtype, int B, cudaStream_t s)
 {
     if (a.Dout > 64 || a.Dout < 1) throw std::runtime_error("pf_kernel: time downsampling must be in [1, 64]");
     // The register kernel wherever its geometry applies, that is for every plan with a time downsampling of 2 to 64
-    // (measured at 2 to 16: 1 beam of rank 10 15 -> 11 us, 8 beams of rank 16 1434 -> 922 us); the general one for a
+    // (measured at 2 to 16: 1 beam of rank 10 15 -> 11 us, 4 beams of rank 16 1434 -> 922 us); the general one for a
     // time downsampling of 1 or above 64.
     if (pf_reg_ok(a)) {
         if (dtype == 0) launch_pf_reg_f32(a, B, s);

@@ -18,7 +18,7 @@
 //
 // What bounds it: instruction issue (83% of the slots; the rows are read from memory once). A kernel that kept the boxcar
 // levels as arrays in shared memory took 47 warp instructions per 32 samples; this one takes 34. Against it, per chunk
-// on a B200 (fp16, 112 trials per output): 8 beams of rank 16 with 5 trees 1434 -> 922 us, 4 beams of rank 12
+// on a B200 (fp16, 112 trials per output): 4 beams of rank 16 with 5 trees 1434 -> 922 us, 16 beams of rank 12
 // 477 -> 362 us; 1 beam of rank 16 in fp32 472 -> 314 us. Registers are held to 5 blocks of 4 warps per SM up to
 // DOUT = 16, 3 and 2 beyond. The last scan reads its window into registers with vector loads: sample by sample from
 // global memory it made the kernel slower than the one it replaces.
