@@ -22,8 +22,10 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # -fmad=false: no fused multiply-add contraction, so the kernels perform the same fp32 roundings as
 # the reference CPU arithmetic they restate.
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-fmad=false", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
-         "--split-compile=4",
          "-Xcudafe", "--diag_suppress=177"]
+# Split compilation changes how nvcc schedules a kernel. The fp32 and fp16 peak finders are 5-8% faster with it (4 beams
+# of rank 16, fp16: 0.98 -> 0.93 ms), the bf16 one 5% slower, and the rank-8 tree kernels 5% slower (1.25 -> 1.33 ms).
+SOURCE_FLAGS = {"pf_reg_f32.cu": ["--split-compile=4"], "pf_reg_f16.cu": ["--split-compile=4"]}
 
 
 def _newest(paths):
@@ -60,7 +62,7 @@ def build(force=False, verbose=False):
 
     def compile_one(src):
         obj = os.path.join(BUILD, src + ".o")
-        cmd = [NVCC] + ARCH + FLAGS + ["-c", os.path.join(CSRC, src), "-o", obj]
+        cmd = [NVCC] + ARCH + FLAGS + SOURCE_FLAGS.get(src, []) + ["-c", os.path.join(CSRC, src), "-o", obj]
         if src.endswith(".cu") and verbose:
             cmd += ["-Xptxas", "-v"]
         r = subprocess.run(cmd, capture_output=True, text=True)
