@@ -267,8 +267,10 @@ struct HaloDims
     static constexpr size_t total = ring + 4 * (M + SEG);
     static_assert(total <= 232448, "shared memory per block");
     static_assert(RPW >= 1 && RPW * NW == NR, "rows per warp");
-    // Blocks per SM that shared memory and a register budget (168 per thread with 16-row trees, 80 below) allow.
-    static constexpr int fit = int(233472 / (total + 1024)), rfit = 65536 / ((RB == 4 ? 168 : 80) * NT);
+    // Blocks per SM that shared memory and a register budget (168 per thread with 16-row trees, 80 below) allow; rank-6
+    // stage 2 runs 2 blocks at 112 registers rather than 3 at 80 (16 rank-12 beams, fp16: 0.280 -> 0.242 ms), rank-6
+    // stage 1 3 (0.224 ms against 0.235).
+    static constexpr int fit = int(233472 / (total + 1024)), rfit = 65536 / ((RB == 4 ? 168 : RB == 3 && STAGE == 2 ? 112 : 80) * NT);
     static constexpr int MINB = fit < rfit ? (fit < 1 ? 1 : fit) : (rfit < 1 ? 1 : rfit);
 };
 

@@ -59,9 +59,10 @@ tree_halo_kernel(const __grid_constant__ typename HaloParamOf<STAGE>::type P)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int b = blockIdx.y, bt = a.beam0 + b;
     const long s0 = a.chunk_ctr ? *a.chunk_ctr * (long) a.nt : a.s0;
-    // The largest power of two up to TILE that divides the chunk (a multiple of 32): every tile then starts at a
-    // multiple of itself, and so do the positions in the delay lines, whose capacities are multiples of it.
-    const int tile = min(TILE, a.nt & -a.nt), ntiles = a.nt / tile;
+    // Tiles of TILE samples, the last one of what remains (a multiple of 32). Output lines never wrap inside a tile: their
+    // capacities are multiples of TILE, or of the chunk where TILE does not divide it. (Equal tiles, of the largest power
+    // of two that divides the chunk, took up to 8% longer on chunks of other lengths.)
+    const int ntiles = (a.nt + TILE - 1) / TILE;
     float *st = a.state + ((long) bt * nblk + blk) * a.state_per_block;
     Ts *st_in = (Ts *) (st + (D::M - TILE * NR));
     const HaloTab<RA, RB> &tab = c_halo_tab<RA, RB>;
@@ -128,14 +129,16 @@ tree_halo_kernel(const __grid_constant__ typename HaloParamOf<STAGE>::type P)
 
     // Copies the next tile of this warp's input rows behind their lookback, 16 bytes per copy, consecutive
     // lanes on consecutive chunks of a row.
-    const int lch = 31 - __clz(tile / EPC);   // log2 of the chunks per tile
-    auto issue = [&]() {
+    constexpr int NCH = TILE / EPC;   // chunks per whole tile
+    auto issue = [&](int next) {
+        const int ch = min(TILE, a.nt - next * TILE) / EPC;
         if constexpr (STAGE == 1) {
-            for (int i = lane; i < (D::RPW << lch); i += 32) {
-                const int r = row0 + (i >> lch), k = i & ((1 << lch) - 1);
-                cp_async_bytes<16>(stg + halo_row<D>(r) + LBK + k * EPC, in + (long) r * a.in_row_stride + pos1 + k * EPC);
+            for (int i = lane; i < D::RPW * NCH; i += 32) {
+                const int r = row0 + i / NCH, k = i % NCH;
+                if (k < ch)
+                    cp_async_bytes<16>(stg + halo_row<D>(r) + LBK + k * EPC, in + (long) r * a.in_row_stride + ((pos1 + k * EPC) & a.in_mask));
             }
-            pos1 = int((pos1 + tile) & a.in_mask);
+            pos1 = int((pos1 + TILE) & a.in_mask);
         } else {
             // One chunk more than the tile, from p & ~(EPC - 1); capacities are multiples of 32 samples, so a
             // chunk never straddles the end of a line and wraps at most once.
@@ -145,19 +148,20 @@ tree_halo_kernel(const __grid_constant__ typename HaloParamOf<STAGE>::type P)
                 q = (q >= t.y) ? q - t.y : q;
                 cp_async_bytes<16>(stg + halo_row<D>(r) + LBK + k * EPC, in + ((long) t.w << 32 | (unsigned) t.z) + q);
             };
-            for (int i = lane; i < (D::RPW << lch); i += 32) copy(row0 + (i >> lch), i & ((1 << lch) - 1));
-            for (int r = row0 + lane; r < row0 + D::RPW; r += 32) copy(r, 1 << lch);
+            for (int i = lane; i < D::RPW * NCH; i += 32)
+                if (i % NCH < ch) copy(row0 + i / NCH, i % NCH);
+            for (int r = row0 + lane; r < row0 + D::RPW; r += 32) copy(r, ch);
             __syncwarp();
             for (int r = row0 + lane; r < row0 + D::RPW; r += 32) {
                 const int4 t = in_tab[r];
-                const int x = t.x + tile;
+                const int x = t.x + TILE;
                 in_tab[r].x = (x >= t.y) ? x - t.y : x;
             }
             __syncwarp();
         }
         cp_async_commit();
     };
-    issue();
+    issue(0);
 
     // Stage 2: multiplet 0 of this thread's coarse dm (d = tid / TL), at its samples of the tile.
     Ts *pf_rows = nullptr;
@@ -165,7 +169,7 @@ tree_halo_kernel(const __grid_constant__ typename HaloParamOf<STAGE>::type P)
     if constexpr (STAGE == 2) {
         const int pf_dm = brev_bits(tid / TL, RA);
         const long rowbase = ((long) bt * a.ndm_out + ((long) brev_bits(blk, a.amb_rank) << RA) + pf_dm) * a.M;
-        pf_rows = (Ts *) a.pf + rowbase * a.pf_cap + kHaloW * (tid % TL);
+        pf_rows = (Ts *) a.pf + rowbase * a.pf_cap;
         pf_slot = int(s0 & (a.pf_cap - 1));
     }
 
@@ -180,17 +184,18 @@ tree_halo_kernel(const __grid_constant__ typename HaloParamOf<STAGE>::type P)
             cp_async_commit();
             T = 0;
         }
+        const int len = min(TILE, a.nt - it * TILE);
         float *ring = ring0 + T;
         cp_async_wait0();
         __syncthreads();
         if constexpr (STAGE == 1) {
-            halo_phase_a<D, 0>(tid, tile, 0, stg, ring, tabw);
+            halo_phase_a<D, 0>(tid, len, 0, stg, ring, tabw);
         } else {
             switch (RA < 2 ? 0 : dm & 3) {
-            case 0: halo_phase_a<D, 0>(tid, tile, dm, stg, ring, tabw); break;
-            case 1: halo_phase_a<D, 1>(tid, tile, dm, stg, ring, tabw); break;
-            case 2: halo_phase_a<D, 2>(tid, tile, dm, stg, ring, tabw); break;
-            default: halo_phase_a<D, 3>(tid, tile, dm, stg, ring, tabw); break;
+            case 0: halo_phase_a<D, 0>(tid, len, dm, stg, ring, tabw); break;
+            case 1: halo_phase_a<D, 1>(tid, len, dm, stg, ring, tabw); break;
+            case 2: halo_phase_a<D, 2>(tid, len, dm, stg, ring, tabw); break;
+            default: halo_phase_a<D, 3>(tid, len, dm, stg, ring, tabw); break;
             }
         }
         __syncthreads();
@@ -201,7 +206,7 @@ tree_halo_kernel(const __grid_constant__ typename HaloParamOf<STAGE>::type P)
 #pragma unroll
             for (int j = 0; j < PL; j++) {
                 const int i = lane + 32 * j;
-                if (i < NV) x[j] = *(const uint4 *) (stg + halo_row<D>(row0 + i / (LBK / EPC)) + tile + i % (LBK / EPC) * EPC);
+                if (i < NV) x[j] = *(const uint4 *) (stg + halo_row<D>(row0 + i / (LBK / EPC)) + len + i % (LBK / EPC) * EPC);
             }
 #pragma unroll
             for (int j = 0; j < PL; j++) {
@@ -210,29 +215,29 @@ tree_halo_kernel(const __grid_constant__ typename HaloParamOf<STAGE>::type P)
             }
             __syncwarp();
         }
-        if (it + 1 < ntiles) issue();
+        if (it + 1 < ntiles) issue(it + 1);
         if constexpr (STAGE == 1) {
             if (tid < NR) {
-                opos = (opos + tile == oend) ? oend - ocap : opos + tile;
+                opos = (opos + TILE == oend) ? oend - ocap : opos + TILE;
                 outpos[((it + 1) & 1) * NR + (tid & (NA - 1)) * NB + (tid >> RA)] = opos;
             }
             Ts *o = out + kHaloW * (tid % TL);
             const int *op = outpos + (it & 1) * NR + (tid / TL) * NB;
-            halo_phase_b<D>(tid, tile, ring, tabr, [&](int f, const float (&x)[4]) { halo_store4(o + halo_tab<NB>(op, f), x); });
+            halo_phase_b<D>(tid, len, ring, tabr, [&](int f, const float (&x)[4]) { halo_store4(o + halo_tab<NB>(op, f), x); });
         } else {
-            Ts *o = pf_rows + pf_slot;
+            Ts *o = pf_rows + ((pf_slot + kHaloW * (tid % TL)) & int(a.pf_cap - 1));
             auto emit = [&](int m, const float (&x)[4]) { halo_store4(o + (long) m * a.pf_cap, x); };
             if constexpr (SUB) {
-                halo_phase_b_sub<D>(tid, tile, ring, tabr, a.sb_count, a.sb_mbase, emit);
+                halo_phase_b_sub<D>(tid, len, ring, tabr, a.sb_count, a.sb_mbase, emit);
             } else {
-                halo_phase_b<D>(tid, tile, ring, tabr, [&](int f, const float (&x)[4]) {
+                halo_phase_b<D>(tid, len, ring, tabr, [&](int f, const float (&x)[4]) {
                     // the full band's multiplet of output row f
                     emit(2 * bitrev_c(f & (NB / 2 - 1), RB - 1) + (f >= NB / 2 ? 1 : 0), x);
                 });
             }
-            pf_slot = int((pf_slot + tile) & (a.pf_cap - 1));
+            pf_slot = int((pf_slot + TILE) & (a.pf_cap - 1));
         }
-        T += tile;
+        T += len;
     }
 
     // Windows and lookback back to the state (the windows are only read in phase b, the lookback is this
