@@ -365,19 +365,23 @@ class PfAvarApproximation:
 _TORCH_DTYPES = {0: "float32", 1: "float16", 2: "bfloat16"}
 
 
+class _DeviceMemory:
+    """A CUDA array interface over memory owned by the dedisperser."""
+    __slots__ = ("__cuda_array_interface__",)
+
+
+_TYPESTR = {"float32": "<f4", "float16": "<f2", "bfloat16": "<i2", "int32": "<i4", "uint8": "|u1"}
+
+
 def _device_tensor(ptr, shape, dtype, device):
     """Wraps device memory owned by the dedisperser as a torch tensor (no copy)."""
     import torch
-    tdt = getattr(torch, dtype)
-    n = int(np.prod(shape))
-    esize = torch.tensor([], dtype=tdt).element_size()
-    if n == 0:
-        return torch.empty(shape, dtype=tdt, device=device)
-    # Build a byte view via the CUDA array interface, then reinterpret.
-    holder = type("_Holder", (), {})()
-    holder.__cuda_array_interface__ = {"shape": (n * esize,), "typestr": "|u1", "data": (int(ptr), False), "version": 3}
-    t = torch.as_tensor(holder, device=device)
-    return t.view(tdt).view(*shape)
+    if 0 in shape:
+        return torch.empty(shape, dtype=getattr(torch, dtype), device=device)
+    mem = _DeviceMemory()
+    mem.__cuda_array_interface__ = {"shape": shape, "typestr": _TYPESTR[dtype], "data": (int(ptr), False), "version": 3}
+    t = torch.as_tensor(mem, device=device)
+    return t.view(torch.bfloat16) if dtype == "bfloat16" else t   # the interface has no bfloat16
 
 
 class Outputs:
