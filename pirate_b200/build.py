@@ -14,7 +14,7 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libpirate_b200.so")
 
-SOURCES = ["plan.cpp", "avar.cpp", "simpulse.cpp", "capi.cpp", "kernels.cu", "tree_halo_f32.cu", "tree_halo_f16.cu", "tree_halo_bf16.cu", "pf_reg_f32.cu", "pf_reg_f16.cu", "pf_reg_bf16.cu", "dedisperser.cu", "noalloc.cu", "sifter.cu", "batched.cu"]
+SOURCES = ["plan.cpp", "avar.cpp", "simpulse.cpp", "capi.cpp", "kernels.cu", "tree_halo_f32.cu", "tree_halo_f16.cu", "tree_halo_bf16.cu", "pf_reg_f32.cu", "pf_reg_f16.cu", "pf_reg_bf16.cu", "pf_reg_main_f32.cu", "pf_reg_main_f16.cu", "pf_reg_main_bf16.cu", "dedisperser.cu", "noalloc.cu", "sifter.cu", "batched.cu"]
 HEADERS = ["plan.hpp", "avar.hpp", "simpulse.hpp", "yaml_lite.hpp", "kernels.cuh", "devutil.cuh", "tree_halo.cuh", "tree_halo_kernel.cuh", "pf_reg.cuh", "dedisperser.hpp", "regtree.cuh", "sifter.hpp", "batched.hpp"]
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
@@ -23,9 +23,10 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # the reference CPU arithmetic they restate.
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-fmad=false", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
          "-Xcudafe", "--diag_suppress=177"]
-# Split compilation changes how nvcc schedules a kernel. The fp32 and fp16 peak finders are 5-8% faster with it (4 beams
-# of rank 16, fp16: 0.98 -> 0.93 ms), the bf16 one 5% slower, and the rank-8 tree kernels 5% slower (1.25 -> 1.33 ms).
-SOURCE_FLAGS = {"pf_reg_f32.cu": ["--split-compile=4"], "pf_reg_f16.cu": ["--split-compile=4"]}
+# Split compilation changes how nvcc schedules a kernel. The peak finder of the widest searches is 3-6% faster with it
+# (4 beams of rank 16, fp16: 0.956 -> 0.924 ms; fp32, 1 beam: 0.338 -> 0.318) and has a source of its own, because beside
+# other kernels the outcome varied more (alone, one build in five came out as without it). The rank-8 tree kernels are 5% slower with it.
+SOURCE_FLAGS = {src: ["--split-compile=4"] for src in ("pf_reg_main_f32.cu", "pf_reg_main_f16.cu", "pf_reg_main_bf16.cu")}
 
 
 def _newest(paths):

@@ -2,8 +2,8 @@
 //
 // One warp per (beam, 32 output times) of one coarse dm, or of 2 or 4 coarse dms where a chunk has at most 16 or 8
 // output times; a lane owns one output time, i.e. DOUT consecutive samples of every multiplet row. Per multiplet
-// the window (the lanes' samples and the tpad before them) is staged in shared memory with cp.async, one multiplet
-// ahead; a lane reads its own DOUT samples and keeps every boxcar level's entries of them in registers. The
+// the window (the lanes' samples and the tpad before them) is staged in shared memory with cp.async, one to
+// three multiplets ahead; a lane reads its own DOUT samples and keeps every boxcar level's entries of them in registers. The
 // entries that a profile reaches back to belong to the lanes before and come by shuffle: the lane that holds the
 // wanted entry offers it, and the entries before the warp's first output time ("halo") are computed by the last
 // lanes of the warp, which offer them in place of their own, since nobody reads those at that distance.
@@ -43,6 +43,9 @@ struct PfReg
     static constexpr int U = BB < 16 ? 16 / BB : 1;                       // lanes per 16-byte chunk
     static constexpr int HL = ((TP + DOUT - 1) / DOUT + U - 1) / U * U;   // halo lanes
     static constexpr int CPL = BB >= 16 ? BB / 16 : 1;                    // chunks per lane
+    // Staged multiplets: 3 ahead where a few blocks wait for their loads (4 rank-11 beams, bf16, in two batches: 210 ->
+    // 180 us; 16 rank-12 beams 362 -> 355 us), 1 ahead for 64 bytes and more a lane (fp32, DOUT 16: 319 us, 323 with 3).
+    static constexpr int NBUF = BB <= 32 ? 4 : 2;
     static constexpr int LWMIN = HL <= 8 ? 8 : HL <= 16 ? 16 : 32;        // fewest lanes per coarse dm
     static_assert(HL <= 32, "halo lanes");
     __host__ __device__ static constexpr int dt(int l) { return (1 << l) < DC ? (1 << l) : DC; }
@@ -317,18 +320,21 @@ __global__ void __launch_bounds__(kPfRegWarps * 32, DOUT <= 16 ? 5 : DOUT == 32 
     const long s0 = a.chunk_ctr ? *a.chunk_ctr * (long) a.nt_chunk : a.s0;
     const int slot0 = int((s0 + (long) tout0 * DOUT) & mask);   // first sample of the warp's first output time
 
-    // Two staging buffers per sub-group, of the LW + HL blocks of DOUT samples.
+    // NBUF staging buffers per sub-group, of the LW + HL blocks of DOUT samples.
     const int wbytes = (LW + HL) * BB;
-    unsigned char *win0 = pfr_sm + (warp * G + sub) * 2 * wbytes;
+    unsigned char *win0 = pfr_sm + (warp * G + sub) * R::NBUF * wbytes;
     const int nch = ((ntw + HL) * BB + 15) / 16;
     auto stage = [&](int m) {
-        const Ts *row = pfrows + (long) m * a.pf_cap;
-        unsigned char *dst = win0 + (m & 1) * wbytes;
-        for (int c = lane; c < nch; c += LW)
-            cp_async_bytes<16>(dst + 16 * R::swz(c), row + ((slot0 - HL * DOUT + c * int(16 / sizeof(Ts))) & mask));
+        if (m < a.M) {
+            const Ts *row = pfrows + (long) m * a.pf_cap;
+            unsigned char *dst = win0 + (m & (R::NBUF - 1)) * wbytes;
+            for (int c = lane; c < nch; c += LW)
+                cp_async_bytes<16>(dst + 16 * R::swz(c), row + ((slot0 - HL * DOUT + c * int(16 / sizeof(Ts))) & mask));
+        }
         cp_async_commit();
     };
-    stage(0);
+#pragma unroll
+    for (int m = 0; m < R::NBUF - 1; m++) stage(m);
 
     float bl[L];
     int ml[L];
@@ -339,11 +345,11 @@ __global__ void __launch_bounds__(kPfRegWarps * 32, DOUT <= 16 ? 5 : DOUT == 32 
     bool pos = false;
 
     for (int m = 0; m < a.M; m++) {
-        // Wait for this multiplet's samples; then stage the next one into the other buffer (every lane is past
-        // its reads of that buffer: they came before the previous iteration's shuffles).
-        cp_async_wait0();
+        // Wait for this multiplet's samples (the newer NBUF - 2 may be in flight); then stage another one into the buffer
+        // of the previous multiplet, which every lane has read: the iteration ended with a warp barrier.
+        cp_async_wait<R::NBUF - 2>();
         __syncwarp();
-        if (m + 1 < a.M) stage(m + 1);
+        stage(m + R::NBUF - 1);
         const int n = a.m_to_n[m];
         if (n != wn) {
             bool ok = true;
@@ -355,7 +361,7 @@ __global__ void __launch_bounds__(kPfRegWarps * 32, DOUT <= 16 ? 5 : DOUT == 32 
             pos = __all_sync(0xffffffffu, ok);
             wn = n;
         }
-        const unsigned char *win = win0 + (m & 1) * wbytes;
+        const unsigned char *win = win0 + (m & (R::NBUF - 1)) * wbytes;
         float e[2][DOUT], h[2][DOUT];
         pfr_load<Ts, L, DOUT>(win, HL + lane, e[0]);
         // Halo: the last HL lanes hold the blocks before the first output time, block HL - k in lane LW - k.
@@ -398,12 +404,19 @@ static void launch_pf_reg(const PfArgs &a, int B, cudaStream_t s)
     int LW = 32;
     while (LW > R::LWMIN && LW / 2 >= a.nt_out) LW /= 2;
     const int G = 32 / LW;
-    const size_t sm = (size_t) kPfRegWarps * G * 2 * (LW + R::HL) * R::BB;
+    const size_t sm = (size_t) kPfRegWarps * G * R::NBUF * (LW + R::HL) * R::BB;
     const dim3 grid((a.nt_out + LW - 1) / LW, (a.ndm_out + kPfRegWarps * G - 1) / (kPfRegWarps * G), B);
     set_smem(pf_reg_kernel<Ts, L, DOUT>, sm);
     pf_reg_kernel<Ts, L, DOUT><<<grid, kPfRegWarps * 32, sm, s>>>(a, LW);
     check_launch("pf_reg_kernel");
 }
+
+// The benchmark's widths and time downsampling, in a translation unit of its own (pf_reg_main_*.cu): it is
+// compiled with other flags (build.py).
+template<typename Ts> void launch_pf_reg_5_16(const PfArgs &a, int B, cudaStream_t s);
+template<> void launch_pf_reg_5_16<float>(const PfArgs &a, int B, cudaStream_t s);
+template<> void launch_pf_reg_5_16<__half>(const PfArgs &a, int B, cudaStream_t s);
+template<> void launch_pf_reg_5_16<__nv_bfloat16>(const PfArgs &a, int B, cudaStream_t s);
 
 template<typename Ts, int L>
 static void launch_pf_reg_d(const PfArgs &a, int B, cudaStream_t s)
@@ -412,7 +425,10 @@ static void launch_pf_reg_d(const PfArgs &a, int B, cudaStream_t s)
     case 2: launch_pf_reg<Ts, L, 2>(a, B, s); break;
     case 4: launch_pf_reg<Ts, L, 4>(a, B, s); break;
     case 8: launch_pf_reg<Ts, L, 8>(a, B, s); break;
-    case 16: launch_pf_reg<Ts, L, 16>(a, B, s); break;
+    case 16:
+        if constexpr (L == 5) launch_pf_reg_5_16<Ts>(a, B, s);
+        else launch_pf_reg<Ts, L, 16>(a, B, s);
+        break;
     case 32: launch_pf_reg<Ts, L, 32>(a, B, s); break;
     case 64: launch_pf_reg<Ts, L, 64>(a, B, s); break;
     default: throw std::runtime_error("pf_reg_kernel: unsupported time downsampling");

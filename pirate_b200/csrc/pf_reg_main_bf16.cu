@@ -1,0 +1,9 @@
+// pf_reg_main_bf16.cu -- the register peak finder for bfloat16 storage, widths to 32 and a time downsampling of 16.
+
+#include "pf_reg.cuh"
+
+namespace pb2 {
+
+template<> void launch_pf_reg_5_16<__nv_bfloat16>(const PfArgs &a, int B, cudaStream_t s) { launch_pf_reg<__nv_bfloat16, 5, 16>(a, B, s); }
+
+}  // namespace pb2
