@@ -2,7 +2,6 @@
 
 #include "sifter.hpp"
 
-#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -117,14 +116,19 @@ void launch_mask_scores(const float *logits, const int *valid, float *scores, in
 // its K loop of 32-wide steps unpipelined, took about 24 launches and 620 us per training step of 512, and 0.4 ms for
 // the 8 candidates of a chunk; these take 3 launches and about 120 us with the host's part, and 38 us with the patches.)
 //   layer1_kernel  Z1 = X W1^T + b1, H1 = bf16(relu(Z1)): 32 x 32 tiles, K in chunks of 64 through a cp.async
-//                  pipeline, split over the blocks of a cluster where a small batch has few tiles
+//                  pipeline
 //   head_kernel    16 candidates per block: layers 2 and 3, and in training everything between the logits and
-//                  the two large weight gradients (loss, g2, g1, partial bias and W3 gradients)
-//   wgrad_kernel   dW1 = g1^T X and dW2 = g2^T H1 in 64 x 64 tiles, with the Adam step in the epilogue
+//                  the weight gradients (loss terms, g, g2, g1)
+//   wgrad_kernel   dW1 = g1^T X, dW2 = g2^T H1 and dW3 = g^T H2 in 64 x 64 tiles, the bias gradients and the loss,
+//                  with the Adam step in the epilogue
+// Every product is one chain of k16 steps from K = 0 and every bias gradient one chain over the candidates, whatever
+// the batch size: a hidden value near a rounding boundary of bf16 rounds another way after another order of its sum, so
+// a candidate's score would depend on the batch that it is scored in, and a training run on the split chosen.
 
 constexpr int kIn = kMlpIn, kH1 = kMlpH1, kH2 = kMlpH2;
 constexpr int kKc = 64, kKPitch = kKc + 8;    // K chunk; padded row of a staged tile (ldmatrix without bank conflicts)
-constexpr int kStages = 3;
+constexpr int kStages = 3;                    // wgrad_kernel
+constexpr int kL1Stages = 5;                  // layer1_kernel: its 27 chunks are a serial chain; 46 KB of shared memory
 constexpr int kHeadRows = 16;
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
@@ -187,21 +191,16 @@ struct Layer1Args
     uint16_t *h;
 };
 
-// Grid (kH1 / 32, row blocks, S) in clusters of the S blocks of one tile; block z sums the K chunks
-// [27 z / S, 27 (z + 1) / S), and the blocks of a cluster then add each other's tiles in rank order.
+// Grid (kH1 / 32, row blocks). The sum over K is not split over blocks (see above).
 __global__ void __launch_bounds__(128) layer1_kernel(Layer1Args g)
 {
-    namespace cg = cooperative_groups;
-    cg::cluster_group cl = cg::this_cluster();
-    __shared__ __align__(16) uint16_t As[kStages][32][kKPitch], Bs[kStages][32][kKPitch];
-    __shared__ float red[32][33];
+    __shared__ __align__(16) uint16_t As[kL1Stages][32][kKPitch], Bs[kL1Stages][32][kKPitch];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n0 = blockIdx.x * 32, m0 = blockIdx.y * 32, z = blockIdx.z, S = gridDim.z;
+    const int n0 = blockIdx.x * 32, m0 = blockIdx.y * 32;
     constexpr int NC = kIn / kKc;
-    const int c0 = NC * z / S, c1 = NC * (z + 1) / S;
     auto load = [&](int c) {
-        if (c < c1) {
-            const int st = c % kStages;
+        if (c < NC) {
+            const int st = c % kL1Stages;
 #pragma unroll
             for (int j = 0; j < 2; j++) {
                 const int i = tid + 128 * j, r = i >> 3, k = (i & 7) * 8;
@@ -212,14 +211,14 @@ __global__ void __launch_bounds__(128) layer1_kernel(Layer1Args g)
         }
         cp_commit();
     };
-    for (int c = c0; c < c0 + kStages - 1; c++) load(c);
+    for (int c = 0; c < kL1Stages - 1; c++) load(c);
     const int wm = (warp >> 1) * 16, wn = (warp & 1) * 16;
     float acc[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
-    for (int c = c0; c < c1; c++) {
-        cp_wait<kStages - 2>();
+    for (int c = 0; c < NC; c++) {
+        cp_wait<kL1Stages - 2>();
         __syncthreads();
-        load(c + kStages - 1);   // into the buffer that was read before this barrier
-        const int st = c % kStages;
+        load(c + kL1Stages - 1);   // into the buffer that was read before this barrier
+        const int st = c % kL1Stages;
 #pragma unroll
         for (int ks = 0; ks < kKc; ks += 16) {
             uint32_t a[4], b[4];
@@ -234,29 +233,16 @@ __global__ void __launch_bounds__(128) layer1_kernel(Layer1Args g)
 #pragma unroll
     for (int t = 0; t < 2; t++)
 #pragma unroll
-        for (int q = 0; q < 4; q++)
-            red[wm + (lane >> 2) + (q >> 1) * 8][wn + t * 8 + (lane & 3) * 2 + (q & 1)] = acc[t][q];
-    if (S > 1) cl.sync();
-    else __syncthreads();
-    for (int i = 1024 * z / S + tid; i < 1024 * (z + 1) / S; i += 128) {
-        const int r = i >> 5, c = i & 31;
-        if (m0 + r >= g.n) continue;
-        float v = 0.0f;
-        if (S > 1) {
-            for (int k = 0; k < S; k++) v += cl.map_shared_rank(&red[0][0], k)[r * 33 + c];
-        } else {
-            v = red[r][c];
+        for (int h = 0; h < 2; h++) {
+            const int r = m0 + wm + (lane >> 2) + 8 * h, c = n0 + wn + t * 8 + (lane & 3) * 2;
+            if (r >= g.n) continue;
+            const float v0 = acc[t][2 * h] + g.bias[c], v1 = acc[t][2 * h + 1] + g.bias[c + 1];
+            *(float2 *) (g.z + (long) r * kH1 + c) = make_float2(v0, v1);
+            *(uint32_t *) (g.h + (long) r * kH1 + c) = uint32_t(bf_bits(relu(v0))) | (uint32_t(bf_bits(relu(v1))) << 16);
         }
-        v += g.bias[n0 + c];
-        const long o = (long) (m0 + r) * kH1 + n0 + c;
-        g.z[o] = v;
-        g.h[o] = bf_bits(relu(v));
-    }
-    if (S > 1) cl.sync();   // no block ends while another reads its tile
 }
 
-// Partial sums of a head block: db1 [0, 256), db2 [256, 384), dW3 [384, 512), db3 512, loss 513.
-constexpr int kPart = kH1 + 2 * kH2 + 2;
+constexpr int kGPitch = 8;   // bf16 per row of the operand gb: g, then zeros (one 16-byte copy)
 
 struct HeadArgs
 {
@@ -265,8 +251,10 @@ struct HeadArgs
     int n;
     float *logits;           // inference
     const float *labels;     // training (null: inference)
-    uint16_t *g1, *g2;       // bf16 (n, kH1), (n, kH2)
-    float *part;             // (blocks, kPart)
+    // Training: gradients of the logits, Z2 and Z1 in fp32 (n), (n, kH2), (n, kH1) for the bias gradients, and rounded
+    // to bf16 as the products take them; H2 as an operand; each candidate's loss term.
+    float *g, *g2, *g1, *ls;
+    uint16_t *gb, *g2b, *g1b, *h2;
 };
 
 struct HeadSmem
@@ -274,9 +262,10 @@ struct HeadSmem
     uint16_t h1[kHeadRows][kH1 + 8];
     uint16_t w2[kH2][kH1 + 8];
     float z2[kHeadRows][kH2 + 4];
+    uint16_t h2[kHeadRows][kH2 + 8];
     uint16_t g2[kHeadRows][kH2 + 8];
-    float w3[kH2];
-    float g[kHeadRows], ls[kHeadRows];
+    uint16_t w3[kH2];
+    float g[kHeadRows];
 };
 
 __global__ void __launch_bounds__(256) head_kernel(HeadArgs g)
@@ -295,7 +284,7 @@ __global__ void __launch_bounds__(256) head_kernel(HeadArgs g)
         cp16(&s.w2[r][k], g.w2 + (long) r * kH1 + k, true);
     }
     cp_commit();
-    if (tid < kH2) s.w3[tid] = bf_float(g.w3[tid]);
+    if (tid < kH2) s.w3[tid] = g.w3[tid];
     cp_wait<0>();
     __syncthreads();
     {
@@ -315,60 +304,64 @@ __global__ void __launch_bounds__(256) head_kernel(HeadArgs g)
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 const int c = c0 + t * 8 + (lane & 3) * 2 + (q & 1);
-                s.z2[(lane >> 2) + (q >> 1) * 8][c] = acc[t][q] + g.b2[c];
+                const int r = (lane >> 2) + (q >> 1) * 8;
+                const float z = acc[t][q] + g.b2[c];
+                s.z2[r][c] = z;
+                s.h2[r][c] = bf_bits(relu(z));
             }
     }
     __syncthreads();
-    // logit = H2 W3^T + b3: 16 threads per row
-    const int row = tid >> 4, part = tid & 15;
-    float v = 0.0f;
+    if (warp == 0) {
+        // logit = H2 W3^T + b3: one tile, W3 its first column
+        float acc[4] = {0, 0, 0, 0};
 #pragma unroll
-    for (int j = 0; j < kH2 / 16; j++) {
-        const int c = part + 16 * j;
-        v += bf_round(relu(s.z2[row][c])) * s.w3[c];
-    }
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const float logit = v + g.b3[0];
-    const bool live = r0 + row < g.n;
-    if (!g.labels) {
-        if (part == 0 && live) g.logits[r0 + row] = logit;
-        return;
-    }
-    // Mean binary cross-entropy; g = (sigmoid(z) - y) / n
-    if (part == 0) {
-        float gi = 0.0f, l = 0.0f;
-        if (live) {
-            const float y = g.labels[r0 + row];
-            const float sig = 1.0f / (1.0f + expf(-logit));
-            gi = (sig - y) / (float) g.n;
-            l = fmaxf(logit, 0.0f) - logit * y + log1pf(expf(-fabsf(logit)));
+        for (int ks = 0; ks < kH2; ks += 16) {
+            uint32_t a[4], b[2] = {0, 0};
+            ldsm4(a, &s.h2[lane & 15][ks + (lane >> 4) * 8]);
+            if (lane < 4) {
+                b[0] = *(const uint32_t *) &s.w3[ks + lane * 2];
+                b[1] = *(const uint32_t *) &s.w3[ks + 8 + lane * 2];
+            }
+            mma_bf16(acc, a, b[0], b[1]);
         }
-        s.g[row] = gi;
-        s.ls[row] = l;
+        if ((lane & 3) == 0) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int row = (lane >> 2) + 8 * h, r = r0 + row;
+                const bool live = r < g.n;
+                const float logit = acc[2 * h] + g.b3[0];
+                if (!g.labels) {
+                    if (live) g.logits[r] = logit;
+                    continue;
+                }
+                // Mean binary cross-entropy; g = (sigmoid(z) - y) / n
+                float gi = 0.0f;
+                if (live) {
+                    const float y = g.labels[r];
+                    const float sig = 1.0f / (1.0f + expf(-logit));
+                    gi = (sig - y) / (float) g.n;
+                    g.g[r] = gi;
+                    *(uint4 *) (g.gb + (long) r * kGPitch) = make_uint4(bf_bits(gi), 0, 0, 0);
+                    g.ls[r] = fmaxf(logit, 0.0f) - logit * y + log1pf(expf(-fabsf(logit)));
+                }
+                s.g[row] = bf_round(gi);
+            }
+        }
     }
+    if (!g.labels) return;
     __syncthreads();
-    float *pt = g.part + (long) blockIdx.x * kPart;
-    if (tid < kH2) {
-        // g2 = (g W3) masked by Z2 > 0; column sums over the block's rows for db2 and dW3
-        float db2 = 0.0f, dw3 = 0.0f;
-#pragma unroll
-        for (int r = 0; r < kHeadRows; r++) {
-            const float gr = bf_round(s.g[r]), z = s.z2[r][tid];
-            const float g2 = (z > 0.0f) ? gr * s.w3[tid] : 0.0f;
-            db2 += g2;
-            dw3 += gr * bf_round(relu(z));
-            const uint16_t h = bf_bits(g2);
-            s.g2[r][tid] = h;
-            if (r0 + r < g.n) g.g2[(long) (r0 + r) * kH2 + tid] = h;
+    for (int i = tid; i < kHeadRows * kH2; i += 256) {
+        // g2 = (g W3) masked by Z2 > 0 (a product of two bf16 values is exact in fp32)
+        const int row = i / kH2, c = i % kH2;
+        const float g2 = (s.z2[row][c] > 0.0f) ? s.g[row] * bf_float(s.w3[c]) : 0.0f;
+        const uint16_t h = bf_bits(g2);
+        s.g2[row][c] = h;
+        if (r0 + row < g.n) {
+            const long o = (long) (r0 + row) * kH2 + c;
+            g.g2[o] = g2;
+            g.g2b[o] = h;
+            g.h2[o] = s.h2[row][c];
         }
-        pt[kH1 + tid] = db2;
-        pt[kH1 + kH2 + tid] = dw3;
-    } else if (tid == kH2) {
-        float db3 = 0.0f, l = 0.0f;
-        for (int r = 0; r < kHeadRows; r++) { db3 += s.g[r]; l += s.ls[r]; }
-        pt[kH1 + 2 * kH2] = db3;
-        pt[kH1 + 2 * kH2 + 1] = l;
     }
     __syncthreads();
     // g1 = (g2 W2) masked by Z1 > 0: warp w takes 32 columns
@@ -391,33 +384,26 @@ __global__ void __launch_bounds__(256) head_kernel(HeadArgs g)
     }
 #pragma unroll
     for (int t = 0; t < 4; t++) {
-        float cs[2] = {0.0f, 0.0f};
         const int c = c0 + t * 8 + (lane & 3) * 2;
 #pragma unroll
         for (int hh = 0; hh < 2; hh++) {
             const int r = r0 + (lane >> 2) + hh * 8;
             if (r < g.n) {
-                const float2 z = *(const float2 *) (g.z1 + (long) r * kH1 + c);
+                const long o = (long) r * kH1 + c;
+                const float2 z = *(const float2 *) (g.z1 + o);
                 const float v0 = (z.x > 0.0f) ? acc[t][2 * hh] : 0.0f, v1 = (z.y > 0.0f) ? acc[t][2 * hh + 1] : 0.0f;
-                cs[0] += v0;
-                cs[1] += v1;
-                *(uint32_t *) (g.g1 + (long) r * kH1 + c) = uint32_t(bf_bits(v0)) | (uint32_t(bf_bits(v1)) << 16);
+                *(float2 *) (g.g1 + o) = make_float2(v0, v1);
+                *(uint32_t *) (g.g1b + o) = uint32_t(bf_bits(v0)) | (uint32_t(bf_bits(v1)) << 16);
             }
         }
-#pragma unroll
-        for (int o = 4; o < 32; o <<= 1) {
-            cs[0] += __shfl_xor_sync(0xffffffffu, cs[0], o);
-            cs[1] += __shfl_xor_sync(0xffffffffu, cs[1], o);
-        }
-        if (lane < 4) { pt[c] = cs[0]; pt[c + 1] = cs[1]; }
     }
 }
 
 struct WgradArgs
 {
-    const uint16_t *g1, *g2, *h1, *x;   // bf16 (n, kH1), (n, kH2), (n, kH1); fp16 (n, kIn)
-    const float *part;
-    int n, nparts, aligned;
+    const uint16_t *g1b, *g2b, *gb, *h1, *h2, *x;   // bf16 (n, kH1), (n, kH2), (n, kGPitch), (n, kH1), (n, kH2); fp16 (n, kIn)
+    const float *g1, *g2, *g, *ls;
+    int n, aligned;
     float *loss;
     float *grad;                        // null: Adam step instead
     float *w, *m, *v;                   // fp32 parameters and moments
@@ -447,32 +433,81 @@ __device__ __forceinline__ void take_grad(const WgradArgs &g, long i, long ib, f
 }
 
 constexpr int kWgK = 32;                             // candidates per pipeline step
-constexpr int kWgTiles1 = (kMlpH1 / 64) * (kMlpIn / 64), kWgTiles2 = (kMlpH2 / 64) * (kMlpH1 / 64);
+constexpr int kWgTiles1 = (kMlpH1 / 64) * (kMlpIn / 64), kWgTiles2 = (kMlpH2 / 64) * (kMlpH1 / 64), kWgTiles3 = kMlpH2 / 64;
+constexpr int kWgTiles = kWgTiles1 + kWgTiles2 + kWgTiles3;
+constexpr int kWgBias = kMlpH1 / 128 + kMlpH2 / 128 + 1;   // blocks of 128 bias gradients, and one for db3 and the loss
+static_assert(kMlpH1 % 128 == 0 && kMlpH2 % 128 == 0, "bias blocks");
+
+// Sum over the candidates of x[i * pitch], in order; the next 32 are loaded while 32 are added.
+__device__ __forceinline__ float chain_sum(const float *x, long pitch, int n)
+{
+    float v = 0.0f, a[32], b[32];
+    auto load = [&](float (&o)[32], int i0) {
+#pragma unroll
+        for (int i = 0; i < 32; i++) o[i] = (i0 + i < n) ? x[(long) (i0 + i) * pitch] : 0.0f;
+    };
+    load(a, 0);
+    for (int i0 = 0; i0 < n; i0 += 32) {
+        load(b, i0 + 32);
+#pragma unroll
+        for (int i = 0; i < 32; i++) {
+            v += a[i];
+            a[i] = b[i];
+        }
+    }
+    return v;
+}
+
+// Bias gradients and the loss (block 'blk' of kWgBias).
+__device__ __forceinline__ void wgrad_bias(const WgradArgs &g, int blk, int tid)
+{
+    constexpr int N1 = kMlpH1 / 128, N2 = kMlpH2 / 128;
+    if (blk < N1) {
+        take_grad(g, oB1 + blk * 128 + tid, -1, chain_sum(g.g1 + blk * 128 + tid, kH1, g.n));
+        return;
+    }
+    if (blk < N1 + N2) {
+        blk -= N1;
+        take_grad(g, oB2 + blk * 128 + tid, -1, chain_sum(g.g2 + blk * 128 + tid, kH2, g.n));
+        return;
+    }
+    // db3 by the last warp; the loss as a sum per 32 candidates, then over those (at most 1024 candidates).
+    __shared__ float red[32];
+    const int lane = tid & 31, warp = tid >> 5;
+    for (int q = warp; q < 32; q += 4) {
+        float v = (q * 32 + lane < g.n) ? g.ls[q * 32 + lane] : 0.0f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) red[q] = v;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        float v = red[lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) g.loss[0] = v / (float) g.n;
+    } else if (tid == 96) {
+        take_grad(g, oB3, -1, chain_sum(g.g, 1, g.n));
+    }
+}
 
 // C(m, c) = sum_k A[k][m] B[k][c] over the n candidates, 64 x 64 tiles, four warps of 32 x 32; operands are read
-// as they lie (candidates in rows) and transposed by ldmatrix. The last block reduces the head blocks' partials.
+// as they lie (candidates in rows) and transposed by ldmatrix. dW3 is row 0 of its tiles.
 __global__ void __launch_bounds__(128) wgrad_kernel(WgradArgs g)
 {
     __shared__ __align__(16) uint16_t As[kStages][kWgK][kKPitch], Bs[kStages][kWgK][kKPitch];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int blk = blockIdx.x;
-    if (blk == kWgTiles1 + kWgTiles2) {
-        for (int i = tid; i < kPart; i += 128) {
-            float v = 0.0f;
-            for (int p = 0; p < g.nparts; p++) v += g.part[(long) p * kPart + i];
-            if (i < kH1) take_grad(g, oB1 + i, -1, v);
-            else if (i < kH1 + kH2) take_grad(g, oB2 + i - kH1, -1, v);
-            else if (i < kH1 + 2 * kH2) take_grad(g, oW3 + i - kH1 - kH2, bW3 + i - kH1 - kH2, v);
-            else if (i == kH1 + 2 * kH2) take_grad(g, oB3, -1, v);
-            else g.loss[0] = v / (float) g.n;
-        }
+    if (blk >= kWgTiles) {
+        wgrad_bias(g, blk - kWgTiles, tid);
         return;
     }
-    const bool first = blk < kWgTiles1;
-    if (!first) blk -= kWgTiles1;
-    const int lda = first ? kH1 : kH2, ldb = first ? kIn : kH1;
+    const bool first = blk < kWgTiles1, third = blk >= kWgTiles1 + kWgTiles2;
+    blk -= first ? 0 : third ? kWgTiles1 + kWgTiles2 : kWgTiles1;
+    const int lda = first ? kH1 : third ? kGPitch : kH2, ldb = first ? kIn : third ? kH2 : kH1;
     const int tn = ldb / 64, m0 = blk / tn * 64, c0 = blk % tn * 64;
-    const uint16_t *A = first ? g.g1 : g.g2, *B = first ? g.x : g.h1;
+    const int na = third ? kGPitch : 64;   // columns of A in memory; zeros beyond
+    const uint16_t *A = first ? g.g1b : third ? g.gb : g.g2b, *B = first ? g.x : third ? g.h2 : g.h1;
     const bool al = first ? g.aligned : true;
     const int nk = (g.n + kWgK - 1) / kWgK;
     auto load = [&](int c) {
@@ -483,7 +518,7 @@ __global__ void __launch_bounds__(128) wgrad_kernel(WgradArgs g)
                 const int i = tid + 128 * j, r = i >> 3, k = (i & 7) * 8;
                 const bool ok = c * kWgK + r < g.n;
                 const long rr = ok ? c * kWgK + r : 0;
-                cp16(&As[st][r][k], A + rr * lda + m0 + k, ok);
+                cp16(&As[st][r][k], A + rr * lda + (k < na ? m0 + k : 0), ok && k < na);
                 copy8(&Bs[st][r][k], B + rr * ldb + c0 + k, ok, al);
             }
         }
@@ -524,15 +559,16 @@ __global__ void __launch_bounds__(128) wgrad_kernel(WgradArgs g)
                 }
         }
     }
-    const long o = first ? oW1 : oW2, ob = first ? bW1 : bW2;
+    const long o = first ? oW1 : third ? oW3 : oW2, ob = first ? bW1 : third ? bW3 : bW2;
 #pragma unroll
     for (int i = 0; i < 2; i++)
 #pragma unroll
         for (int t = 0; t < 4; t++)
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                const long e = (long) (m0 + wm + i * 16 + (lane >> 2) + (q >> 1) * 8) * ldb + c0 + wn + t * 8 + (lane & 3) * 2 + (q & 1);
-                take_grad(g, o + e, ob + e, acc[i][t][q]);
+                const int m = m0 + wm + i * 16 + (lane >> 2) + (q >> 1) * 8;
+                const long e = (long) m * ldb + c0 + wn + t * 8 + (lane & 3) * 2 + (q & 1);
+                if (!third || m == 0) take_grad(g, o + e, ob + e, acc[i][t][q]);
             }
 }
 
@@ -561,9 +597,14 @@ Sifter::Sifter(int device_, long max_batch_, uint64_t seed) : device(device_), m
     SF_CHECK(cudaMalloc(&z1, max_batch * kMlpH1 * sizeof(float)));
     SF_CHECK(cudaMalloc(&loss, sizeof(float)));
     SF_CHECK(cudaMalloc(&h1, max_batch * kMlpH1 * sizeof(uint16_t)));
-    SF_CHECK(cudaMalloc(&g1, max_batch * kMlpH1 * sizeof(uint16_t)));
-    SF_CHECK(cudaMalloc(&g2, max_batch * kMlpH2 * sizeof(uint16_t)));
-    SF_CHECK(cudaMalloc(&part, blocks(max_batch, kHeadRows) * kPart * sizeof(float)));
+    SF_CHECK(cudaMalloc(&h2, max_batch * kMlpH2 * sizeof(uint16_t)));
+    SF_CHECK(cudaMalloc(&g, max_batch * sizeof(float)));
+    SF_CHECK(cudaMalloc(&ls, max_batch * sizeof(float)));
+    SF_CHECK(cudaMalloc(&g1, max_batch * kMlpH1 * sizeof(float)));
+    SF_CHECK(cudaMalloc(&g2, max_batch * kMlpH2 * sizeof(float)));
+    SF_CHECK(cudaMalloc(&gb, max_batch * kGPitch * sizeof(uint16_t)));
+    SF_CHECK(cudaMalloc(&g1b, max_batch * kMlpH1 * sizeof(uint16_t)));
+    SF_CHECK(cudaMalloc(&g2b, max_batch * kMlpH2 * sizeof(uint16_t)));
     SF_CHECK(cudaFuncSetAttribute(head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(HeadSmem)));
     SF_CHECK(cudaMemset(adam_m, 0, kNparams * sizeof(float)));
     SF_CHECK(cudaMemset(adam_v, 0, kNparams * sizeof(float)));
@@ -584,7 +625,8 @@ Sifter::~Sifter()
 {
     cudaSetDevice(device);
     for (void *q : {(void *) master, (void *) grad, (void *) adam_m, (void *) adam_v, (void *) wb, (void *) z1,
-                    (void *) loss, (void *) h1, (void *) g1, (void *) g2, (void *) part})
+                    (void *) loss, (void *) ls, (void *) h1, (void *) h2, (void *) g, (void *) g1, (void *) g2, (void *) gb,
+                    (void *) g1b, (void *) g2b})
         if (q) cudaFree(q);
 }
 
@@ -620,22 +662,8 @@ void Sifter::layer1(const uint16_t *patches, long n, cudaStream_t s)
     a.aligned = (reinterpret_cast<uintptr_t>(patches) & 15) == 0;   // a patch is 3456 bytes
     a.z = z1;
     a.h = h1;
-    // Split K until about one block per SM has work: the tiles are 32 x 32 of n x 256, 8 per 32 candidates, and a
-    // block's 27 K steps are a serial chain.
-    const long tiles = (kMlpH1 / 32) * blocks(n, 32);
-    const unsigned S = tiles <= 18 ? 8 : tiles <= 37 ? 4 : tiles <= 74 ? 2 : 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kMlpH1 / 32, blocks(n, 32), S);
-    cfg.blockDim = dim3(128);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 1;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = S;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    SF_CHECK(cudaLaunchKernelEx(&cfg, layer1_kernel, a));
+    layer1_kernel<<<dim3(kMlpH1 / 32, blocks(n, 32)), 128, 0, s>>>(a);
+    sf_check_launch("layer1_kernel");
 }
 
 void Sifter::forward(const uint16_t *patches, long n, float *logits, cudaStream_t s)
@@ -646,7 +674,7 @@ void Sifter::forward(const uint16_t *patches, long n, float *logits, cudaStream_
     head(n, logits, nullptr, s);
 }
 
-// Layers 2 and 3 of the batch in h1: the logits, or with labels the loss, g2, g1 and the partial gradients.
+// Layers 2 and 3 of the batch in h1: the logits, or with labels the loss terms and the gradients of the logits, Z2 and Z1.
 void Sifter::head(long n, float *logits, const float *labels, cudaStream_t s)
 {
     HeadArgs a;
@@ -659,9 +687,14 @@ void Sifter::head(long n, float *logits, const float *labels, cudaStream_t s)
     a.n = int(n);
     a.logits = logits;
     a.labels = labels;
-    a.g1 = g1;
+    a.g = g;
     a.g2 = g2;
-    a.part = part;
+    a.g1 = g1;
+    a.ls = ls;
+    a.gb = gb;
+    a.g2b = g2b;
+    a.g1b = g1b;
+    a.h2 = h2;
     head_kernel<<<blocks(n, kHeadRows), 256, sizeof(HeadSmem), s>>>(a);
     sf_check_launch("head_kernel");
 }
@@ -674,13 +707,17 @@ void Sifter::train(const uint16_t *patches, const float *labels, long n, bool ad
     layer1(patches, n, s);
     head(n, nullptr, labels, s);
     WgradArgs a;
+    a.g1b = g1b;
+    a.g2b = g2b;
+    a.gb = gb;
+    a.h1 = h1;
+    a.h2 = h2;
+    a.x = patches;
     a.g1 = g1;
     a.g2 = g2;
-    a.h1 = h1;
-    a.x = patches;
-    a.part = part;
+    a.g = g;
+    a.ls = ls;
     a.n = int(n);
-    a.nparts = int(blocks(n, kHeadRows));
     a.aligned = (reinterpret_cast<uintptr_t>(patches) & 15) == 0;
     a.loss = loss;
     a.grad = adam ? nullptr : grad;
@@ -691,7 +728,7 @@ void Sifter::train(const uint16_t *patches, const float *labels, long n, bool ad
     a.lr = lr;
     a.c1 = 1.0f - std::pow(0.9f, float(step));
     a.c2 = 1.0f - std::pow(0.999f, float(step));
-    wgrad_kernel<<<kWgTiles1 + kWgTiles2 + 1, 128, 0, s>>>(a);
+    wgrad_kernel<<<kWgTiles + kWgBias, 128, 0, s>>>(a);
     sf_check_launch("wgrad_kernel");
 }
 

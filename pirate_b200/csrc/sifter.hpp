@@ -94,10 +94,10 @@ private:
     float *grad = nullptr;       // nparams fp32
     float *adam_m = nullptr, *adam_v = nullptr;
     uint16_t *wb = nullptr;      // bf16 copies of W1, W2, W3 (biases stay fp32)
-    float *z1 = nullptr, *loss = nullptr;
-    uint16_t *h1 = nullptr;                  // bf16 activations
-    uint16_t *g2 = nullptr, *g1 = nullptr;   // bf16 gradients of Z2 and Z1 (as the products take them)
-    float *part = nullptr;                   // partial gradients of the biases and W3
+    float *z1 = nullptr, *loss = nullptr, *ls = nullptr;           // ls: loss terms
+    uint16_t *h1 = nullptr, *h2 = nullptr;                         // bf16 activations
+    float *g = nullptr, *g2 = nullptr, *g1 = nullptr;              // gradients of the logits, Z2 and Z1
+    uint16_t *gb = nullptr, *g2b = nullptr, *g1b = nullptr;        // rounded to bf16, as the products take them
     long step = 0;
 };
 
