@@ -371,11 +371,8 @@ void GpuDedisperser::allocate()
                 for (long r = 0; r < pow2(R1); r++) {
                     long row = blk * pow2(R1) + r;
                     if (spill[row]) continue;
-                    // one sample more than the lags need: stage 2 also reads the sample before its first; a
-                    // multiple of the stage-1 kernel's tile, or of the chunk where that is none, so that no tile
-                    // of an output line wraps
-                    const long unit = (st.nt % halo_tile(R1) == 0) ? halo_tile(R1) : st.nt;
-                    cap[row] = cap_r[row] = int(round_up(plan.max_row_lag[p][row] + st.nt + 1, unit));
+                    // one sample more than the lags need: stage 2 also reads the sample before its first
+                    cap[row] = cap_r[row] = int(round_up(plan.max_row_lag[p][row] + st.nt + 1, 32));
                     off[row] = off_r[row] = tot;
                     tot += cap[row];
                 }

@@ -260,11 +260,12 @@ struct HaloDims
     static constexpr int SU = NORM ? 0 : RA + RB;                 // unnormalized steps of an output
     static constexpr size_t tabw = 0;                             // int[NR]: phase-a store offsets, [f][d]
     static constexpr size_t tabr = tabw + 4 * NR;                 // int[NR]: phase-b load offsets, [d][f]
-    static constexpr size_t outpos = tabr + 4 * NR;               // int[2][NR]: stage 1, output positions, [d][f]
+    static constexpr int PARTS = TILE / 32, PSTR = NR + 8;        // 8: a warp's parts lie in different banks
+    static constexpr size_t outpos = tabr + 4 * NR;               // int[PARTS][PSTR]: stage 1, output positions, [d][f]
     static constexpr size_t in_tab = tabr + 4 * NR;               // int4[NR]: stage 2, input rows
-    static constexpr size_t stg = (tabr + 4 * NR + (STAGE == 1 ? 8 : 16) * NR + 127) & ~size_t(127);
+    static constexpr size_t stg = (tabr + 4 * NR + (STAGE == 1 ? 4 * PARTS * PSTR : 16 * NR) + 127) & ~size_t(127);
     static constexpr size_t ring = (stg + sizeof(Ts) * GSTR * NB + 127) & ~size_t(127);
-    static constexpr size_t total = ring + 4 * (M + SEG);
+    static constexpr size_t total = ring + 4 * (M + SEG - TILE);  // the last tile of a segment starts at SEG - TILE
     static_assert(total <= 232448, "shared memory per block");
     static_assert(RPW >= 1 && RPW * NW == NR, "rows per warp");
     // Blocks per SM that shared memory and a register budget (168 per thread with 16-row trees, 80 below) allow; rank-6

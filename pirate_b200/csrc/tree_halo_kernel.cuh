@@ -59,9 +59,8 @@ tree_halo_kernel(const __grid_constant__ typename HaloParamOf<STAGE>::type P)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int b = blockIdx.y, bt = a.beam0 + b;
     const long s0 = a.chunk_ctr ? *a.chunk_ctr * (long) a.nt : a.s0;
-    // Tiles of TILE samples, the last one of what remains (a multiple of 32). Output lines never wrap inside a tile: their
-    // capacities are multiples of TILE, or of the chunk where TILE does not divide it. (Equal tiles, of the largest power
-    // of two that divides the chunk, took up to 8% longer on chunks of other lengths.)
+    // Tiles of TILE samples, the last one of what remains (a multiple of 32). (Equal tiles, of the largest power of two
+    // that divides the chunk, took up to 8% longer on chunks of other lengths.)
     const int ntiles = (a.nt + TILE - 1) / TILE;
     float *st = a.state + ((long) bt * nblk + blk) * a.state_per_block;
     Ts *st_in = (Ts *) (st + (D::M - TILE * NR));
@@ -91,7 +90,7 @@ tree_halo_kernel(const __grid_constant__ typename HaloParamOf<STAGE>::type P)
 
     const Ts *in;
     int pos1 = 0, dm = 0;               // stage 1: read position of every input row; stage 2: the rows' lag factor
-    int opos = 0, oend = 0, ocap = 0;   // stage 1: thread r's output line (position of the tile, end, capacity)
+    int opos = 0, oend = 0, ocap = 0;   // stage 1: output line [d][f] = tid (next position, end, capacity)
     Ts *out = nullptr;
     if constexpr (STAGE == 1) {
         in = (const Ts *) a.in + (long) (a.in_beam0 + b) * a.in_beam_stride + (long) blk * NR * a.in_row_stride;
@@ -106,16 +105,25 @@ tree_halo_kernel(const __grid_constant__ typename HaloParamOf<STAGE>::type P)
         tabw[r] = A + halo_lb4(F) + F * brev_bits(d, RA);
         tabr[d * NB + f] = A;
     }
+    // Positions of the tile's parts of 32 samples in this thread's output line. Lines hold a multiple of 32 samples, so no
+    // part wraps; a position per tile would need lines of whole tiles or chunks, up to twice the memory for a chunk that
+    // is no multiple of the tile.
+    auto next_outpos = [&]() {
+#pragma unroll
+        for (int j = 0; j < D::PARTS; j++) {
+            outpos[j * D::PSTR + tid] = opos;
+            opos = (opos + 32 == oend) ? oend - ocap : opos + 32;
+        }
+    };
     if constexpr (STAGE == 1) {
         static_assert(D::NT >= NR, "one thread per output line");
         if (tid < NR) {
             // the host checks that a block's lines span < 2^31 samples
-            const long row = (long) blk * NR + tid;
+            const long row = (long) blk * NR + ((tid % NB) << RA) + tid / NB;
             const int off = int(a.ring_off[row] - a.ring_off[(long) blk * NR]);
             ocap = a.ring_cap[row];
             opos = off + int(s0 % ocap);
             oend = off + ocap;
-            outpos[(tid & (NA - 1)) * NB + (tid >> RA)] = opos;   // of tile 0; the tables of even and odd tiles alternate
         }
     } else {
         for (int r = row0 + lane; r < row0 + D::RPW; r += 32) {
@@ -189,6 +197,7 @@ tree_halo_kernel(const __grid_constant__ typename HaloParamOf<STAGE>::type P)
         cp_async_wait0();
         __syncthreads();
         if constexpr (STAGE == 1) {
+            if (tid < NR) next_outpos();
             halo_phase_a<D, 0>(tid, len, 0, stg, ring, tabw);
         } else {
             switch (RA < 2 ? 0 : dm & 3) {
@@ -217,12 +226,9 @@ tree_halo_kernel(const __grid_constant__ typename HaloParamOf<STAGE>::type P)
         }
         if (it + 1 < ntiles) issue(it + 1);
         if constexpr (STAGE == 1) {
-            if (tid < NR) {
-                opos = (opos + TILE == oend) ? oend - ocap : opos + TILE;
-                outpos[((it + 1) & 1) * NR + (tid & (NA - 1)) * NB + (tid >> RA)] = opos;
-            }
-            Ts *o = out + kHaloW * (tid % TL);
-            const int *op = outpos + (it & 1) * NR + (tid / TL) * NB;
+            constexpr int PV = 32 / kHaloW;   // threads per part
+            Ts *o = out + kHaloW * (tid % PV);
+            const int *op = outpos + (tid % TL / PV) * D::PSTR + (tid / TL) * NB;
             halo_phase_b<D>(tid, len, ring, tabr, [&](int f, const float (&x)[4]) { halo_store4(o + halo_tab<NB>(op, f), x); });
         } else {
             Ts *o = pf_rows + ((pf_slot + kHaloW * (tid % TL)) & int(a.pf_cap - 1));

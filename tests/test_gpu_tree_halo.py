@@ -59,3 +59,17 @@ def test_tree_tiles_16bit(pb2lib, dtype, tol):
     for seq in range(4):
         for i in range(orc.ntrees):
             assert np.abs(gres[seq][0][i] - ores[seq][0][i]).max() <= tol
+
+
+def test_delay_lines_need_no_whole_chunks(pb2lib):
+    """Delay lines hold a multiple of 32 samples at every chunk length: 64 samples more per chunk cost 64/2048 more
+    memory, also where the chunk is then no multiple of the kernel's tile (128 samples at dd rank 6)."""
+    size = {}
+    for nt in (2048, 2112):
+        cfg = H.toy_config(rank=12, nfreq=1024, nt=nt, dtype="float16", subbands=[0, 0, 0, 1], beams_per_gpu=1, beams_per_batch=1,
+                           primary_trees=[dict(num_early_triggers=0, max_width=8, dm_downsampling=0, time_downsampling=0,
+                                               wt_dm_downsampling=64, wt_time_downsampling=16)])
+        dd = pb2lib.GpuDedisperser(pb2lib.DedispersionPlan(pb2lib.DedispersionConfig.from_dict(cfg)))
+        dd.allocate()
+        size[nt] = dd.device_bytes()
+    assert size[2112] <= 1.04 * size[2048]
