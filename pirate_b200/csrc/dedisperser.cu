@@ -371,8 +371,9 @@ void GpuDedisperser::allocate()
                 for (long r = 0; r < pow2(R1); r++) {
                     long row = blk * pow2(R1) + r;
                     if (spill[row]) continue;
-                    // one sample more than the lags need: stage 2 also reads the sample before its first
-                    cap[row] = cap_r[row] = int(round_up(plan.max_row_lag[p][row] + st.nt + 1, 32));
+                    // The lags' reach and the chunk. Stage 2 reads whole 16-byte pieces, so up to 7 samples before its
+                    // first; chunks start at multiples of 32 samples, so those lie within the rounding.
+                    cap[row] = cap_r[row] = int(round_up(plan.max_row_lag[p][row] + st.nt, 32));
                     off[row] = off_r[row] = tot;
                     tot += cap[row];
                 }
