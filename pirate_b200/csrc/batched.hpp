@@ -7,7 +7,7 @@
 // parallel branches (or one serial chain), and replayed every chunk. Every kernel reads the chunk index
 // from a device counter that the graph's last node advances, so the same executable graph serves every
 // chunk without parameter updates. A project autotuner times the schedule choices (per group: merged or
-// per-tree stage-2 grids, peak-finding kernel variant, gridding block size; and branch concurrency)
+// per-tree stage-2 grids, peak-finding kernel variant, block size of grid_lds_kernel; and branch concurrency)
 // with CUDA events on the replayed graph and keeps the fastest.
 
 #pragma once

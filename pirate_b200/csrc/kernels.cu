@@ -1108,22 +1108,19 @@ template<typename Ts, int NLEV>
 static void launch_grid_lds_t(const GridLdsArgs &a, cudaStream_t s)
 {
     if (a.q_data && a.T % 256) throw std::runtime_error("grid_lds_kernel: int4 input needs a chunk length that is a multiple of 256");
-    if constexpr (NLEV <= 4) {
+    if (grid_warp_ok(a.T, NLEV)) {
         // A warp per pair for whole steps, faster than a thread per window at every size measured (1 beam of rank 10
         // 11 -> 10 us, of rank 8 the same; larger ones above grid_warp_kernel). 16-sample windows where the levels need
         // them, and for int4 input, whose tables then have two scale blocks per step for the warp to fill.
-        if (a.T % 512 == 0 && (a.q_data || NLEV == 4)) {
+        if constexpr (NLEV == 4) {
             if (a.q_data) launch_grid_warp<Ts, NLEV, 16, true>(a, s);
-            else if constexpr (NLEV == 4) launch_grid_warp<Ts, NLEV, 16, false>(a, s);
-            return;
+            else launch_grid_warp<Ts, NLEV, 16, false>(a, s);
+        } else if constexpr (NLEV < 4) {
+            if (!a.q_data) launch_grid_warp<Ts, NLEV, 8, false>(a, s);
+            else if (a.T % 512 == 0) launch_grid_warp<Ts, NLEV, 16, true>(a, s);
+            else launch_grid_warp<Ts, NLEV, 8, true>(a, s);
         }
-        if constexpr (NLEV < 4) {
-            if (a.T % 256 == 0) {
-                if (a.q_data) launch_grid_warp<Ts, NLEV, 8, true>(a, s);
-                else launch_grid_warp<Ts, NLEV, 8, false>(a, s);
-                return;
-            }
-        }
+        return;
     }
     constexpr int W0 = ((1 << NLEV) > 8) ? (1 << NLEV) : 8;
     if (a.T % W0) throw std::runtime_error("grid_lds_kernel: chunk length not a multiple of the window");

@@ -172,6 +172,9 @@ struct SpillArgs
 void launch_spill_g2h(const SpillArgs &a, cudaStream_t s);
 void launch_spill_h2g(const SpillArgs &a, cudaStream_t s);
 
+// Whether grid_warp_kernel grids chunks of T samples with nlev downsampled levels (else grid_lds_kernel, which alone has a
+// block size to choose): whole steps of 32 windows, of 8 samples, or 16 with four levels.
+inline bool grid_warp_ok(long T, int nlev) { return nlev < 4 ? T % 256 == 0 : nlev == 4 && T % 512 == 0; }
 void launch_grid_lds(const GridLdsArgs &a, int dtype, cudaStream_t s);
 // int4 -> out_dtype dequantization of (nbeams, nfreq, ntime) samples (ntime a multiple of 256).
 void launch_dequantize(void *out, int out_dtype, const void *data, const void *scales_offsets, long nbeams, long nfreq,

@@ -74,3 +74,31 @@ def test_batched_graph_matches_oracle_and_autotune(pb2lib):
     bd.set_schedule([False] * 3, [True] * 3, [256] * 3, concurrent=False)
     bd.reset()
     check(_run(bd, cfgs, xs, nchunks), "serial, unmerged, general peak finder")
+
+
+def test_grid_block_is_tried_where_it_has_an_effect(pb2lib):
+    """Chunks that are no multiple of 256 samples are gridded by grid_lds_kernel: its block size is a schedule choice,
+    and every choice gives the same bits. Where grid_warp_kernel runs there is none, and the autotuner tries none."""
+    pb = pb2lib
+    tries = {}
+    for nt in (384, 512):
+        cfg = H.toy_config(rank=8, nfreq=200, nt=nt, subbands=[1], beams_per_gpu=2, beams_per_batch=2,
+                           primary_trees=H._prim(8, [(0, 8, 0), (0, 4, 0)], 16))
+        bd = pb.BatchedDedisperser([pb.DedispersionPlan(pb.DedispersionConfig.from_dict(cfg))], cuda_device_id=0)
+        bd.allocate()
+        x = H.make_inputs(cfg, 3, seed=6)
+        orc, _ = H.run_oracle(cfg, [], [])
+        ws = H.make_weights(orc, seed=7)
+        for i, w in enumerate(ws):
+            bd.fill_all_weights(0, i, w)
+        _, ores = H.run_oracle(cfg, x, ws, 1, 32)
+        for block in (32, 96, 256, 512) if nt == 384 else (128,):
+            bd.set_schedule([True], [False], [block])
+            bd.reset()
+            res = _run(bd, [cfg], [x], 3)
+            for c in range(3):
+                for i in range(len(ores[c][0])):
+                    assert np.array_equal(res[c][0][0][i], ores[c][0][i]) and np.array_equal(res[c][0][1][i], ores[c][1][i]), (block, c, i)
+        bd.set_schedule([True], [False], [128])
+        tries[nt] = [t["try"] for t in bd.autotune(reps=1)["candidates"]]
+    assert tries[384].count("grid_block") == 3 and tries[512].count("grid_block") == 0
