@@ -14,7 +14,7 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libpirate_b200.so")
 
-SOURCES = ["plan.cpp", "avar.cpp", "simpulse.cpp", "capi.cpp", "kernels.cu", "tree_halo_f32.cu", "tree_halo_f16.cu", "tree_halo_bf16.cu", "pf_reg_f32.cu", "pf_reg_f16.cu", "pf_reg_bf16.cu", "pf_reg_main_f32.cu", "pf_reg_main_f16.cu", "pf_reg_main_bf16.cu", "dedisperser.cu", "noalloc.cu", "sifter.cu", "batched.cu"]
+SOURCES = ["plan.cpp", "avar.cpp", "simpulse.cpp", "capi.cpp", "kernels.cu", "tree_halo_f32.cu", "tree_halo_f16.cu", "tree_halo_bf16.cu", "pf_reg_f32.cu", "pf_reg_f16.cu", "pf_reg_bf16.cu", "dedisperser.cu", "noalloc.cu", "sifter.cu", "batched.cu"]
 HEADERS = ["plan.hpp", "avar.hpp", "simpulse.hpp", "yaml_lite.hpp", "kernels.cuh", "devutil.cuh", "tree_halo.cuh", "tree_halo_kernel.cuh", "pf_reg.cuh", "dedisperser.hpp", "regtree.cuh", "sifter.hpp", "batched.hpp"]
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
@@ -23,10 +23,8 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # the reference CPU arithmetic they restate.
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-fmad=false", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
          "-Xcudafe", "--diag_suppress=177"]
-# Split compilation changes how nvcc schedules a kernel. The peak finder of the widest searches is 3-6% faster with it
-# (4 beams of rank 16, fp16: 0.956 -> 0.924 ms; fp32, 1 beam: 0.338 -> 0.318) and has a source of its own, because beside
-# other kernels the outcome varied more (alone, one build in five came out as without it). The rank-8 tree kernels are 5% slower with it.
-SOURCE_FLAGS = {src: ["--split-compile=4"] for src in ("pf_reg_main_f32.cu", "pf_reg_main_f16.cu", "pf_reg_main_bf16.cu")}
+# No --split-compile: with it the code that nvcc makes of one source differs from build to build, and its speed with it
+# (the peak finder of 4 rank-16 beams 0.925 or 0.979 ms; the rank-8 tree kernels 5% slower).
 
 
 def _newest(paths):
@@ -63,7 +61,7 @@ def build(force=False, verbose=False):
 
     def compile_one(src):
         obj = os.path.join(BUILD, src + ".o")
-        cmd = [NVCC] + ARCH + FLAGS + SOURCE_FLAGS.get(src, []) + ["-c", os.path.join(CSRC, src), "-o", obj]
+        cmd = [NVCC] + ARCH + FLAGS + ["-c", os.path.join(CSRC, src), "-o", obj]
         if src.endswith(".cu") and verbose:
             cmd += ["-Xptxas", "-v"]
         r = subprocess.run(cmd, capture_output=True, text=True)

@@ -1247,8 +1247,8 @@ void launch_pf(const PfArgs &a, int dtype, int B, cudaStream_t s)
 {
     if (a.Dout > 64 || a.Dout < 1) throw std::runtime_error("pf_kernel: time downsampling must be in [1, 64]");
     // The register kernel wherever its geometry applies, that is for every plan with a time downsampling of 2 to 64
-    // (measured at 2 to 16: 1 beam of rank 10 15 -> 11 us, 4 beams of rank 16 1434 -> 922 us); the general one for a
-    // time downsampling of 1 or above 64.
+    // (measured at 2 to 16: 1 beam of rank 10 15 -> 11 us, 4 beams of rank 16 1434 -> 957 us); the general one for a
+    // time downsampling of 1.
     if (pf_reg_ok(a)) {
         if (dtype == 0) launch_pf_reg_f32(a, B, s);
         else if (dtype == 1) launch_pf_reg_f16(a, B, s);

@@ -18,8 +18,8 @@
 //
 // What bounds it: instruction issue (83% of the slots; the rows are read from memory once). A kernel that kept the boxcar
 // levels as arrays in shared memory took 47 warp instructions per 32 samples; this one takes 34. Against it, per chunk
-// on a B200 (fp16, 112 trials per output): 4 beams of rank 16 with 5 trees 1434 -> 922 us, 16 beams of rank 12
-// 477 -> 362 us; 1 beam of rank 16 in fp32 472 -> 314 us. Registers are held to 5 blocks of 4 warps per SM up to
+// on a B200 (fp16, 112 trials per output): 4 beams of rank 16 with 5 trees 1434 -> 957 us, 16 beams of rank 12
+// 477 -> 355 us; 1 beam of rank 16 in fp32 472 -> 338 us. Registers are held to 5 blocks of 4 warps per SM up to
 // DOUT = 16, 3 and 2 beyond. The last scan reads its window into registers with vector loads: sample by sample from
 // global memory it made the kernel slower than the one it replaces.
 
@@ -44,7 +44,7 @@ struct PfReg
     static constexpr int HL = ((TP + DOUT - 1) / DOUT + U - 1) / U * U;   // halo lanes
     static constexpr int CPL = BB >= 16 ? BB / 16 : 1;                    // chunks per lane
     // Staged multiplets: 3 ahead where a few blocks wait for their loads (4 rank-11 beams, bf16, in two batches: 210 ->
-    // 180 us; 16 rank-12 beams 362 -> 355 us), 1 ahead for 64 bytes and more a lane (fp32, DOUT 16: 319 us, 323 with 3).
+    // 180 us; 16 rank-12 beams 362 -> 355 us), 1 ahead for 64 bytes and more a lane (fp32, DOUT 16: 338 us, 346 with 3).
     static constexpr int NBUF = BB <= 32 ? 4 : 2;
     static constexpr int LWMIN = HL <= 8 ? 8 : HL <= 16 ? 16 : 32;        // fewest lanes per coarse dm
     static_assert(HL <= 32, "halo lanes");
@@ -411,13 +411,6 @@ static void launch_pf_reg(const PfArgs &a, int B, cudaStream_t s)
     check_launch("pf_reg_kernel");
 }
 
-// The benchmark's widths and time downsampling, in a translation unit of its own (pf_reg_main_*.cu): it is
-// compiled with other flags (build.py).
-template<typename Ts> void launch_pf_reg_5_16(const PfArgs &a, int B, cudaStream_t s);
-template<> void launch_pf_reg_5_16<float>(const PfArgs &a, int B, cudaStream_t s);
-template<> void launch_pf_reg_5_16<__half>(const PfArgs &a, int B, cudaStream_t s);
-template<> void launch_pf_reg_5_16<__nv_bfloat16>(const PfArgs &a, int B, cudaStream_t s);
-
 template<typename Ts, int L>
 static void launch_pf_reg_d(const PfArgs &a, int B, cudaStream_t s)
 {
@@ -425,10 +418,7 @@ static void launch_pf_reg_d(const PfArgs &a, int B, cudaStream_t s)
     case 2: launch_pf_reg<Ts, L, 2>(a, B, s); break;
     case 4: launch_pf_reg<Ts, L, 4>(a, B, s); break;
     case 8: launch_pf_reg<Ts, L, 8>(a, B, s); break;
-    case 16:
-        if constexpr (L == 5) launch_pf_reg_5_16<Ts>(a, B, s);
-        else launch_pf_reg<Ts, L, 16>(a, B, s);
-        break;
+    case 16: launch_pf_reg<Ts, L, 16>(a, B, s); break;
     case 32: launch_pf_reg<Ts, L, 32>(a, B, s); break;
     case 64: launch_pf_reg<Ts, L, 64>(a, B, s); break;
     default: throw std::runtime_error("pf_reg_kernel: unsupported time downsampling");
