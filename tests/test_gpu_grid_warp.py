@@ -1,7 +1,8 @@
 """Gridding and lagged downsampling by a warp per channel pair, at the edges: fewer pairs than a block has warps, chunks
 of one step and of several, split over blocks or carried from step to step, 0 to 4 downsampled levels in 8- and 16-sample
 windows, input channels per tree channel from a fraction to dozens, and int4 input with and without the tables. float32
-outputs must equal the fp32 oracle's bit for bit; int4 input must give what the dequantized samples give."""
+outputs must equal the fp32 oracle's bit for bit; int4 input must give what the dequantized samples give; chunks that
+the kernel does not take must give what the same stream gives in chunks that it takes."""
 
 import numpy as np
 import pytest
@@ -71,3 +72,19 @@ def test_grid_warp_int4(pb2lib, dtype, nt, npri, nfreq):
                 outs += [t.clone() for t in out.out_max + out.out_argmax]
         res.append(outs)
     assert all(torch.equal(a, b) for a, b in zip(*res))
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float16", "bfloat16"])
+def test_grid_lds_same_as_grid_warp(pb2lib, dtype):
+    """A stream in chunks of 384 samples (a thread per window, with a downsampled level) and of 768 (a warp per pair)."""
+    rng = np.random.default_rng(9)
+    x = rng.standard_normal((2, 100, 4 * 768)).astype(np.float32)
+    res = []
+    for nt in (384, 768):
+        cfg = _cfg(8, 100, nt, 2, 2, dtype)
+        orc, _ = H.run_oracle(cfg, [], [])
+        ws = H.make_weights(orc, seed=1, kind="bare")
+        _, _, g = H.run_gpu(pb2lib, cfg, [np.ascontiguousarray(x[:, :, k:k + nt]) for k in range(0, x.shape[2], nt)], ws)
+        res.append([np.concatenate([r[k][i] for r in g], axis=-1) for k in (0, 1) for i in range(orc.ntrees)])
+    for a, b in zip(*res):
+        assert np.array_equal(a, b)

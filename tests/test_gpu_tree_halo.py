@@ -1,8 +1,8 @@
 """The tree kernels at the edges of their tiles: float32 outputs must equal the fp32 oracle's bit for bit.
 
-Tiles are the largest power of two up to 64-256 samples (by tree rank) that divides the chunk, segments 512-2048
-samples; blocks read their rows at every alignment. The cases take chunks of one short tile, of an odd number of
-tiles, longer than a segment, every dd rank from 1 to 8, full-band and (staggered) subband outputs."""
+Tiles are 64 samples at dd ranks 7 and 8, 128 at 6 and 256 below, the last one of a chunk what remains; segments
+512-2048 samples; blocks read their rows at every alignment. The cases take chunks of one short tile, with a short
+last tile, longer than a segment, every dd rank from 1 to 8, full-band and (staggered) subband outputs."""
 
 import numpy as np
 import pytest
@@ -13,14 +13,15 @@ pytestmark = pytest.mark.gpu
 
 # (rank, nt, subbands, primary trees as (early triggers, max width), chunks)
 CASES = [
-    (3, 32, [1], [(0, 4)], 9),                         # dd ranks 1 + 2, one 32-sample tile
-    (4, 96, [0, 1], [(1, 4)], 7),                      # dd ranks 2 + 1, 2; three 32-sample tiles
-    (5, 352, [1, 1], [(2, 8)], 4),                     # dd ranks 2 + 1..3
-    (6, 4160, [0, 0, 1], [(1, 8), (0, 4)], 2),         # 64-sample tiles of long-tile trees, segments of 2048
+    (3, 32, [1], [(0, 4)], 9),                         # dd ranks 1 + 2, one tile of 32 samples
+    (4, 96, [0, 1], [(1, 4)], 7),                      # dd ranks 2 + 1, 2; one tile of 96
+    (5, 352, [1, 1], [(2, 8)], 4),                     # dd ranks 2 + 1..3; a tile and 96 samples
+    (6, 4160, [0, 0, 1], [(1, 8), (0, 4)], 2),         # two segments of 2048 and 64 samples
     (9, 2560, [0, 0, 0, 1], [(0, 16), (0, 8)], 2),     # dd ranks 4, 5: a segment and a quarter
     (10, 448, [4, 7, 3, 1], [(1, 8)], 4),              # every subband level, staggered pairs
-    (12, 192, [0, 3, 0, 1], [(1, 16), (0, 8)], 4),     # dd ranks 5, 6, odd tiles
-    (14, 640, [0, 0, 0, 0, 1], [(0, 8), (0, 4)], 2),   # dd rank 7: segments of 2048 (float32), odd tiles
+    (12, 192, [0, 3, 0, 1], [(1, 16), (0, 8)], 4),     # dd ranks 5, 6; a tile and a half
+    (14, 640, [0, 0, 0, 0, 1], [(0, 8), (0, 4)], 2),   # dd rank 7: ten tiles
+    (14, 2144, [0, 0, 0, 0, 1], [(0, 8)], 2),          # dd rank 7: a float32 segment (2048), a tile and a half
     (16, 1088, [0, 1, 0, 0, 1], [(0, 8)], 2),          # dd rank 8: a float32 segment (1024) and one tile
 ]
 
@@ -73,3 +74,23 @@ def test_delay_lines_need_no_whole_chunks(pb2lib):
         dd.allocate()
         size[nt] = dd.device_bytes()
     assert size[2112] <= 1.04 * size[2048]
+
+
+# (rank, subbands, samples per long chunk): dd ranks 4, 6, 7 and 8; past the 16-bit segments of 2048, 2048, 512 and 2048
+# samples, the last tile partial at dd ranks 4 and 6.
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
+@pytest.mark.parametrize("rank,subbands,nt", [(8, [1, 1, 1], 2112), (12, [0, 1, 0, 1], 2112), (14, [0, 0, 0, 0, 1], 576), (16, [0, 0, 0, 0, 1], 2112)])
+def test_chunk_length_does_not_change_outputs(pb2lib, rank, subbands, nt, dtype):
+    """A stream cut into long chunks gives what it gives cut into chunks of 64 samples, bit for bit."""
+    rng = np.random.default_rng(rank)
+    x = rng.standard_normal((1, 300, 2 * nt)).astype(np.float32)
+    res = []
+    for n in (64, nt):
+        cfg = H.toy_config(rank=rank, nfreq=300, nt=n, dtype=dtype, subbands=subbands, beams_per_gpu=1, beams_per_batch=1,
+                           primary_trees=[dict(num_early_triggers=0, max_width=8, dm_downsampling=0, time_downsampling=0,
+                                               wt_dm_downsampling=2 ** (rank // 2), wt_time_downsampling=16)])
+        orc, _ = H.run_oracle(cfg, [], [])
+        ws = H.make_weights(orc, seed=1, kind="bare")
+        _, _, g = H.run_gpu(pb2lib, cfg, [np.ascontiguousarray(x[:, :, k:k + n]) for k in range(0, 2 * nt, n)], ws)
+        res.append([np.concatenate([r[k][0] for r in g], axis=-1) for k in (0, 1)])
+    assert np.array_equal(res[0][0], res[1][0]) and np.array_equal(res[0][1], res[1][1])
