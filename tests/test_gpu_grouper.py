@@ -76,6 +76,20 @@ def test_beam_peaks_planted(pb2lib, dtype):
     assert got[1][3].item() == -1 and got[0][3].item() == -np.inf
 
 
+@pytest.mark.parametrize("dtype", ["float32", "float16", "bfloat16"])
+@pytest.mark.parametrize("B,shapes", [(2000, [(64, 16)]), (1, [(1, 1)]), (700, [(5, 13), (40, 7)]), (300, [(127, 33), (64, 64)]),
+                                      (3, [(1000, 999)]), (1, [(4096, 128), (3, 1)]), (2, [(513, 32)])])
+def test_beam_peaks_block_sizes(pb2lib, dtype, B, shapes):
+    """From 128 to 1024 threads per block and 1 to 8 blocks per beam, on and off the vector path."""
+    import torch
+    gen = torch.Generator().manual_seed(B)
+    maxes = [torch.randint(-50, 50, (B,) + s, generator=gen).to(getattr(torch, dtype)) for s in shapes]   # many ties
+    args = [np.random.default_rng(1).integers(0, 2 ** 32, size=(B,) + s, dtype=np.uint64).astype(np.uint32) for s in shapes]
+    got = pb2lib.beam_peaks(([m.cuda() for m in maxes], [torch.from_numpy(a.view(np.int32)).cuda() for a in args]))
+    torch.cuda.synchronize()
+    _check(got, toy_peaks_numpy([m.float().numpy() for m in maxes], args))
+
+
 def test_toy_grouper_on_dedisperser_outputs(pb2lib):
     """ToyGrouper over several chunks of a float16 plan with 2 batches: per-beam peaks equal the
     numpy loop on the same outputs, and the events are the thresholded, decoded peaks."""
@@ -111,8 +125,8 @@ def test_toy_grouper_on_dedisperser_outputs(pb2lib):
 
 @pytest.mark.parametrize("dtype", ["float32", "float16"])
 def test_candidate_stage_peaks(pb2lib, dtype):
-    """The candidate stage's split per-beam reduction (many blocks per tree and beam, then one warp per
-    beam) gives the numpy loop's peaks on real outputs, NaN inputs included."""
+    """The candidate stage's per-beam reduction gives the numpy loop's peaks on real outputs, NaN inputs
+    included."""
     import torch
     cfg = H.toy_config(rank=9, nfreq=300, nt=512, dtype=dtype, beams_per_gpu=6, beams_per_batch=6)
     plan = pb2lib.DedispersionPlan(pb2lib.DedispersionConfig.from_dict(cfg))
