@@ -193,7 +193,7 @@ std::string BatchedDedisperser::autotune(int reps)
             if (knob == 0) { auto t = best; t[g].merge_stage2 = !t[g].merge_stage2; alts.push_back(t); }
             if (knob == 1) { auto t = best; t[g].pf_general = !t[g].pf_general; alts.push_back(t); }
             // the gridding block size only where the kernel that has one runs: identical schedules differ by noise
-            if (knob == 2 && !grid_warp_ok(plans[g].nt_in, int(plans[g].num_primary_trees) - 1)) for (int gb : {64, 256, 512}) if (gb != best[g].grid_block) { auto t = best; t[g].grid_block = gb; alts.push_back(t); }
+            if (knob == 2 && !grid_warp_ok(plans[g].nt_in, int(plans[g].num_primary_trees) - 1, plans[g].nfreq, int(plans[g].config.toplevel_tree_rank), false)) for (int gb : {64, 256, 512}) if (gb != best[g].grid_block) { auto t = best; t[g].grid_block = gb; alts.push_back(t); }
             for (auto &t : alts) {
                 double ms = measure(t, best_conc);
                 const char *names[3] = {"merge_stage2", "pf_general", "grid_block"};

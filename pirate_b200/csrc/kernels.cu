@@ -634,6 +634,34 @@ __device__ __forceinline__ float2 f2fma(float2 a, float2 b, float2 c)
     return f2from(d);
 }
 
+__device__ __forceinline__ float2 f2add(float2 a, float2 b)
+{
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(f2bits(a)), "l"(f2bits(b)));
+    return f2from(d);
+}
+
+// W samples of one input row as they lie in memory; zeros when !ok.
+template<typename Ts, int W>
+struct GridRow
+{
+    uint4 q[W * sizeof(Ts) / 16];
+    __device__ __forceinline__ void load(const Ts *p, bool ok)
+    {
+#pragma unroll
+        for (int v = 0; v < int(W * sizeof(Ts) / 16); v++) q[v] = ok ? ((const uint4 *) p)[v] : make_uint4(0, 0, 0, 0);
+    }
+    __device__ __forceinline__ float get(int i) const
+    {
+        constexpr int PER = 16 / sizeof(Ts);
+        const uint4 &u = q[i / PER];
+        const int j = i % PER * int(sizeof(Ts)) / 4;
+        const uint32_t v = j == 0 ? u.x : j == 1 ? u.y : j == 2 ? u.z : u.w;
+        if constexpr (sizeof(Ts) == 4) return __uint_as_float(v);
+        else if constexpr (std::is_same<Ts, __half>::value) return __half2float(__ushort_as_half((unsigned short) (v >> (i & 1) * 16)));
+        else return __uint_as_float((i & 1) ? (v & 0xffff0000u) : (v << 16));
+    }
+};
 // Two samples as one word of a 16-bit type.
 template<typename Ts>
 __device__ __forceinline__ uint32_t pack2(float x, float y)
@@ -789,7 +817,8 @@ __device__ __forceinline__ void lut_words(const unsigned char *p, uint32_t (&q)[
     }
 }
 
-template<typename Ts, int NLEV, int W, bool Q>
+// WIDE: plans with at least as many input channels as tree channels (not for int4).
+template<typename Ts, int NLEV, int W, bool Q, bool WIDE>
 __global__ void __launch_bounds__(32 * kGridWarps, W == 16 ? (Q ? 6 : 5) : 8) grid_warp_kernel(GridLdsArgs a)
 {
     using G = GridWarp<Ts, NLEV, W, Q>;
@@ -859,10 +888,16 @@ __global__ void __launch_bounds__(32 * kGridWarps, W == 16 ? (Q ? 6 : 5) : 8) gr
         float2 r[W];   // the channels' samples: even (x) and odd (y)
         if (use_lut) {
 #pragma unroll 1
-            for (int k = 0; k < rows; k++) {
-                const float2 sc = __half22float2(so[(long) k * (a.T >> 8)]);
-                const float x = (lane & 15) == 8 ? 0.0f : to_f(from_f<Ts>(__fadd_rn(__fmul_rn(sc.x, fv), sc.y)));
-                if (G::NBLK == 2 || lane < 16) ((float *) wsm)[k * G::NBLK * 16 + lane] = x;
+            for (int k = 0; k < rows; k += 2) {
+                __half2 p[2];
+#pragma unroll
+                for (int g = 0; g < 2; g++) p[g] = so[(long) min(k + g, rows - 1) * (a.T >> 8)];
+#pragma unroll
+                for (int g = 0; g < 2; g++) {
+                    const float2 sc = __half22float2(p[g]);
+                    const float x = (lane & 15) == 8 ? 0.0f : to_f(from_f<Ts>(__fadd_rn(__fmul_rn(sc.x, fv), sc.y)));
+                    if (G::NBLK == 2 || lane < 16) ((float *) wsm)[min(k + g, rows - 1) * G::NBLK * 16 + lane] = x;
+                }
             }
             so += G::NBLK;
             __syncwarp();
@@ -874,18 +909,19 @@ __global__ void __launch_bounds__(32 * kGridWarps, W == 16 ? (Q ? 6 : 5) : 8) gr
 #pragma unroll
                 for (int i = 0; i < W; i++) r[i] = make_float2(ca ? r[i].x : 0.0f, cb ? r[i].y : 0.0f);
 #pragma unroll 1
-            for (int k = 1; k < ca; k++) {
-                lut_words<W>(qa + (long) k * (a.T >> 1), va);
-                const float wk = wa[k];
+            for (int k = 1; k < max(ca, cb); k++) {
+                if (k < ca) lut_words<W>(qa + (long) k * (a.T >> 1), va);
+                if (k < cb) lut_words<W>(qb + (long) k * (a.T >> 1), vb);
+                if (k < ca) {
+                    const float wk = wa[k];
 #pragma unroll
-                for (int i = 0; i < W; i++) r[i].x = __fadd_rn(r[i].x, __fmul_rn(wk, lut_at(la + k * G::NBLK * 64, va[i / 8], i & 7)));
-            }
-#pragma unroll 1
-            for (int k = 1; k < cb; k++) {
-                lut_words<W>(qb + (long) k * (a.T >> 1), vb);
-                const float wk = wb[k];
+                    for (int i = 0; i < W; i++) r[i].x = __fadd_rn(r[i].x, __fmul_rn(wk, lut_at(la + k * G::NBLK * 64, va[i / 8], i & 7)));
+                }
+                if (k < cb) {
+                    const float wk = wb[k];
 #pragma unroll
-                for (int i = 0; i < W; i++) r[i].y = __fadd_rn(r[i].y, __fmul_rn(wk, lut_at(lb + k * G::NBLK * 64, vb[i / 8], i & 7)));
+                    for (int i = 0; i < W; i++) r[i].y = __fadd_rn(r[i].y, __fmul_rn(wk, lut_at(lb + k * G::NBLK * 64, vb[i / 8], i & 7)));
+                }
             }
             qa += STEP / 2;
             qb += STEP / 2;
@@ -902,6 +938,32 @@ __global__ void __launch_bounds__(32 * kGridWarps, W == 16 ? (Q ? 6 : 5) : 8) gr
             grid_run<Ts, W, Q>(a, b, 2 * c + 1, t0, x);
 #pragma unroll
             for (int i = 0; i < W; i++) r[i].y = x[i];
+        } else if constexpr (WIDE) {
+            // Both channels' rows together, in pairs where registers allow, so that their loads are in flight together; a
+            // channel past its last row adds 0 * 0.
+            constexpr int GR = W * sizeof(Ts) <= 16 ? 2 : 1;
+            const Ts *pa = (const Ts *) a.in + ((long) b * a.F + fa) * a.T + t0, *pb = pa + (long) (fb - fa) * a.T;
+#pragma unroll
+            for (int i = 0; i < W; i++) r[i] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+            for (int k = 0; k < max(ca, cb); k += GR) {
+                GridRow<Ts, W> x[GR], y[GR];
+                float2 w[GR];
+#pragma unroll
+                for (int g = 0; g < GR; g++) {
+                    const bool oka = k + g < ca, okb = k + g < cb;
+                    w[g] = make_float2(oka ? wa[k + g] : 0.0f, okb ? wb[k + g] : 0.0f);
+                    x[g].load(pa, oka);
+                    y[g].load(pb, okb);
+                    pa += a.T;
+                    pb += a.T;
+                }
+                // Scalar products: a packed product and the packed sum that takes it came out as one fused operation.
+#pragma unroll
+                for (int g = 0; g < GR; g++)
+#pragma unroll
+                    for (int i = 0; i < W; i++) r[i] = f2add(r[i], make_float2(__fmul_rn(w[g].x, x[g].get(i)), __fmul_rn(w[g].y, y[g].get(i))));
+            }
         } else {
             const Ts *in = (const Ts *) a.in + (long) b * a.F * a.T + t0;
             float x[W], y[W];
@@ -1113,9 +1175,21 @@ template<typename Ts, int NLEV, int W, bool Q>
 static void launch_grid_warp(const GridLdsArgs &a, cudaStream_t s)
 {
     const int nblk = ((1 << (a.rank - 1)) + kGridWarps - 1) / kGridWarps, nsteps = a.T / (32 * W);
-    // Few pairs: split the chunk over up to 8 blocks per SM.
-    const int nz = std::max(1, std::min(nsteps, 8 * 148 / std::max(1, nblk * a.B)));
-    grid_warp_kernel<Ts, NLEV, W, Q><<<dim3(nblk, a.B, nz), 32 * kGridWarps, 0, s>>>(a);
+    // Few pairs: split the chunk over up to 8 blocks per SM, or 32 and 64 where a tree channel sums 1 and 4 input
+    // channels and more: those of the low end of the band sum three times the average and are the longest chains.
+    // 8 beams of rank 10, fp16, 3 trees, 1 input channel per tree channel 33 -> 29 us, 4 115 -> 58, 16 407 -> 152, the
+    // rows' loads of WIDE included.
+    const int per_sm = a.F >> a.rank >= 4 ? 64 : a.F >> a.rank >= 1 ? 32 : 8;
+    const int nz = std::max(1, std::min(nsteps, per_sm * 148 / std::max(1, nblk * a.B)));
+    const dim3 grid(nblk, a.B, nz);
+    if constexpr (!Q) {
+        if (a.F >> a.rank >= 1) {
+            grid_warp_kernel<Ts, NLEV, W, Q, true><<<grid, 32 * kGridWarps, 0, s>>>(a);
+            check_launch("grid_warp_kernel");
+            return;
+        }
+    }
+    grid_warp_kernel<Ts, NLEV, W, Q, false><<<grid, 32 * kGridWarps, 0, s>>>(a);
     check_launch("grid_warp_kernel");
 }
 
@@ -1123,9 +1197,9 @@ template<typename Ts, int NLEV>
 static void launch_grid_lds_t(const GridLdsArgs &a, cudaStream_t s)
 {
     if (a.q_data && a.T % 256) throw std::runtime_error("grid_lds_kernel: int4 input needs a chunk length that is a multiple of 256");
-    if (grid_warp_ok(a.T, NLEV)) {
-        // A warp per pair for whole steps, faster than a thread per window at every size measured (1 beam of rank 10
-        // 11 -> 10 us, of rank 8 the same; larger ones above grid_warp_kernel). 16-sample windows where the levels need
+    if (grid_warp_ok(a.T, NLEV, a.F, a.rank, a.q_data != nullptr)) {
+        // A warp per pair for whole steps, faster than a thread per window (1 beam of rank 10 11 -> 10 us, of rank 8 the
+        // same; larger ones above grid_warp_kernel), but for int4 input of many channels (see grid_warp_ok). 16-sample windows where the levels need
         // them, and for int4 input, whose tables then have two scale blocks per step for the warp to fill.
         if constexpr (NLEV == 4) {
             if (a.q_data) launch_grid_warp<Ts, NLEV, 16, true>(a, s);

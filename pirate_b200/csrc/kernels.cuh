@@ -172,9 +172,14 @@ struct SpillArgs
 void launch_spill_g2h(const SpillArgs &a, cudaStream_t s);
 void launch_spill_h2g(const SpillArgs &a, cudaStream_t s);
 
-// Whether grid_warp_kernel grids chunks of T samples with nlev downsampled levels (else grid_lds_kernel, which alone has a
-// block size to choose): whole steps of 32 windows, of 8 samples, or 16 with four levels.
-inline bool grid_warp_ok(long T, int nlev) { return nlev < 4 ? T % 256 == 0 : nlev == 4 && T % 512 == 0; }
+// Whether grid_warp_kernel grids F input channels to 2^rank tree channels in chunks of T samples with nlev downsampled
+// levels (else grid_lds_kernel, which alone has a block size to choose): whole steps of 32 windows, of 8 samples, or 16
+// with four levels; int4 input of 4 and more channels per tree channel has more rows per pair than its tables take
+// (4 beams of rank 12, fp16, five trees, 8 channels: 219 us, 172 us by grid_lds_kernel).
+inline bool grid_warp_ok(long T, int nlev, long F, int rank, bool int4)
+{
+    return (nlev < 4 ? T % 256 == 0 : nlev == 4 && T % 512 == 0) && !(int4 && F >> rank >= 4);
+}
 void launch_grid_lds(const GridLdsArgs &a, int dtype, cudaStream_t s);
 // int4 -> out_dtype dequantization of (nbeams, nfreq, ntime) samples (ntime a multiple of 256).
 void launch_dequantize(void *out, int out_dtype, const void *data, const void *scales_offsets, long nbeams, long nfreq,

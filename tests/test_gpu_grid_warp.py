@@ -74,14 +74,15 @@ def test_grid_warp_int4(pb2lib, dtype, nt, npri, nfreq):
     assert all(torch.equal(a, b) for a, b in zip(*res))
 
 
+@pytest.mark.parametrize("nfreq", [100, 256, 1500])   # up to 1 and 2, 2 to 3, and 2 to 17 input channels per tree channel
 @pytest.mark.parametrize("dtype", ["float32", "float16", "bfloat16"])
-def test_grid_lds_same_as_grid_warp(pb2lib, dtype):
+def test_grid_lds_same_as_grid_warp(pb2lib, dtype, nfreq):
     """A stream in chunks of 384 samples (a thread per window, with a downsampled level) and of 768 (a warp per pair)."""
     rng = np.random.default_rng(9)
-    x = rng.standard_normal((2, 100, 4 * 768)).astype(np.float32)
+    x = rng.standard_normal((2, nfreq, 4 * 768)).astype(np.float32)
     res = []
     for nt in (384, 768):
-        cfg = _cfg(8, 100, nt, 2, 2, dtype)
+        cfg = _cfg(8, nfreq, nt, 2, 2, dtype)
         orc, _ = H.run_oracle(cfg, [], [])
         ws = H.make_weights(orc, seed=1, kind="bare")
         _, _, g = H.run_gpu(pb2lib, cfg, [np.ascontiguousarray(x[:, :, k:k + nt]) for k in range(0, x.shape[2], nt)], ws)
