@@ -40,7 +40,6 @@ namespace pb2 {
 // level in registers, and gets the even channel's predecessor sample at each level by gridding the
 // 2^nlev samples before its window (at the chunk start: from a parity double-buffered state).
 
-
 // Loads W consecutive samples starting at p (16-byte vectors when W*sizeof(Ts) allows; p must then be
 // 16-byte aligned).
 template<typename Ts, int W>
@@ -1021,9 +1020,6 @@ constexpr int kPfWarps = 4;
 // Number of entries of boxcar level l in a window of len0 samples (level 0 = samples).
 __device__ __forceinline__ int pf_nlev(int len0, int l, int dt) { return (len0 - (1 << l)) / dt + 1; }
 
-template<typename Ts>
-__device__ __forceinline__ float ld_f(const Ts *p) { return to_f(*p); }
-
 // Loads multiplet row 'row' over the warp's window into lev[0..len0) and builds boxcar levels
 // 1..L-1 after it with the reference recursion B_{l+1}[u] = B_l[r u] + B_l[r u + s].
 template<typename Ts, int L>
@@ -1166,10 +1162,8 @@ __global__ void __launch_bounds__(kPfWarps * 32) pf_kernel(PfArgs a, int warp_fl
     }
 }
 
-
 // -------------------------------------------------------------------------------------------------
 // Host launchers.
-
 
 template<typename Ts, int NLEV, int W, bool Q>
 static void launch_grid_warp(const GridLdsArgs &a, cudaStream_t s)
@@ -1306,7 +1300,6 @@ int pf_warp_floats(int Dout, int tpad, int Dcore, int L)
     }
     return tot;
 }
-
 
 template<typename Ts, int L>
 static void launch_pf_l(const PfArgs &a, int B, cudaStream_t s)

@@ -32,8 +32,8 @@
 // The delay line between the phases is one shared-memory buffer for all rows: row r's window
 // [T - lb4, T + P + tile) of delayed times u lies at A_r + lb4 + u, the windows back to back, and all windows
 // advance together by one tile, each into the samples its successor has just dropped. So no index wraps: the
-// buffer is kHaloSeg floats longer than the windows, and a chunk longer than that is done in segments that
-// start again at T = 0 from the saved state.
+// buffer has room for HaloDims::SEG samples of that, and a longer chunk is done in segments that start again at
+// T = 0 from the saved state.
 
 #pragma once
 
@@ -43,11 +43,6 @@
 #include <type_traits>
 
 namespace pb2 {
-
-// The tile functions are plain code over pointers: a host program can define PB2_HD to run them on the CPU.
-#ifndef PB2_HD
-#define PB2_HD __device__ __forceinline__
-#endif
 
 // Window offsets A_r of row r = f * 2^RA + d; A[2^(RA+RB)] = M.
 template<int RA, int RB>
@@ -116,20 +111,9 @@ __host__ __device__ constexpr HaloExt<K, W> make_halo_ext_sub()
     return e;
 }
 
-#ifdef __CUDA_ARCH__
-template<bool NORM> PB2_HD float halo_bfly(float x, float y) { return bfly_n<NORM>(x, y); }
-PB2_HD float halo_out(float v, int n) { return tree_out(v, n); }
-PB2_HD float halo_mul(float x) { return __fmul_rn(kRsqrt2, x); }
-#else
-PB2_HD float halo_mul(float x) { return kRsqrt2 * x; }
-template<bool NORM> PB2_HD float halo_bfly(float x, float y) { float s = x + y; return NORM ? kRsqrt2 * s : s; }
-PB2_HD float halo_out(float v, int n) { return n ? v * tree_scale(n) : v; }
-#endif
-
 // Two fp32 additions in one sm_100 packed f32x2 instruction, each rounded to nearest.
-PB2_HD float2 halo_add2(float2 a, float2 b)
+__device__ __forceinline__ float2 halo_add2(float2 a, float2 b)
 {
-#ifdef __CUDA_ARCH__
     unsigned long long x, y, d;
     asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(a.x), "f"(a.y));
     asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(b.x), "f"(b.y));
@@ -137,9 +121,6 @@ PB2_HD float2 halo_add2(float2 a, float2 b)
     float2 r;
     asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(d));
     return r;
-#else
-    return make_float2(a.x + b.x, a.y + b.y);
-#endif
 }
 
 // Index of sample 0 in a row's registers: even, so that even samples start register pairs.
@@ -147,18 +128,18 @@ __host__ __device__ constexpr int halo_org(int K) { return K > 0 ? (1 << K) : 2;
 
 // n[t] = butterfly of x[t - L] and y[t] for t in [lo, hi): even lags two samples at a time.
 template<bool NORM, int W, int O>
-PB2_HD void halo_add(float (&n)[W + O], const float (&x)[W + O], const float (&y)[W + O], int L, int lo, int hi)
+__device__ __forceinline__ void halo_add(float (&n)[W + O], const float (&x)[W + O], const float (&y)[W + O], int L, int lo, int hi)
 {
 #pragma unroll
     for (int t = -O; t < W; t += 2) {
         const bool a = (t >= lo && t < hi), b = (t + 1 >= lo && t + 1 < hi);
         if (a && b && (L & 1) == 0) {
             const float2 s = halo_add2(make_float2(x[t - L + O], x[t + 1 - L + O]), make_float2(y[t + O], y[t + 1 + O]));
-            n[t + O] = NORM ? halo_mul(s.x) : s.x;
-            n[t + 1 + O] = NORM ? halo_mul(s.y) : s.y;
+            n[t + O] = NORM ? __fmul_rn(kRsqrt2, s.x) : s.x;
+            n[t + 1 + O] = NORM ? __fmul_rn(kRsqrt2, s.y) : s.y;
         } else {
-            if (a) n[t + O] = halo_bfly<NORM>(x[t - L + O], y[t + O]);
-            if (b) n[t + 1 + O] = halo_bfly<NORM>(x[t + 1 - L + O], y[t + 1 + O]);
+            if (a) n[t + O] = bfly_n<NORM>(x[t - L + O], y[t + O]);
+            if (b) n[t + 1 + O] = bfly_n<NORM>(x[t + 1 - L + O], y[t + 1 + O]);
         }
     }
 }
@@ -167,7 +148,7 @@ PB2_HD void halo_add(float (&n)[W + O], const float (&x)[W + O], const float (&y
 // then the step that joins them), which keeps the live registers close to the outputs'. load(row) fills
 // v[row][t + O] over the input range. Sample t of a row is v[row][t + O].
 template<int K, int W, bool NORM, int LV, int BASE, typename Load>
-PB2_HD void halo_tree(float (&v)[1 << K][W + halo_org(K)], Load load)
+__device__ __forceinline__ void halo_tree(float (&v)[1 << K][W + halo_org(K)], Load load)
 {
     constexpr HaloExt<K, W> E = make_halo_ext<K, W>();
     constexpr int O = halo_org(K);
@@ -195,7 +176,7 @@ PB2_HD void halo_tree(float (&v)[1 << K][W + halo_org(K)], Load load)
 
 // Four consecutive samples from an address aligned to four samples.
 template<typename Ts>
-PB2_HD void halo_load4(const Ts *p, float (&o)[4])
+__device__ __forceinline__ void halo_load4(const Ts *p, float (&o)[4])
 {
     if constexpr (sizeof(Ts) == 4) {
         const float4 q = *(const float4 *) p;
@@ -219,7 +200,7 @@ PB2_HD void halo_load4(const Ts *p, float (&o)[4])
 }
 
 template<typename Ts>
-PB2_HD void halo_store4(Ts *p, const float (&o)[4])
+__device__ __forceinline__ void halo_store4(Ts *p, const float (&o)[4])
 {
     if constexpr (sizeof(Ts) == 4) {
         *(float4 *) p = make_float4(o[0], o[1], o[2], o[3]);
@@ -277,7 +258,7 @@ struct HaloDims
 
 // Entry i of a table row of N ints (16-byte loads where the row is a multiple of 16 bytes).
 template<int N>
-PB2_HD int halo_tab(const int *row, int i)
+__device__ __forceinline__ int halo_tab(const int *row, int i)
 {
     if constexpr (N % 4 != 0) {
         return row[i];
@@ -288,7 +269,7 @@ PB2_HD int halo_tab(const int *row, int i)
 }
 
 // Offset of staged row r (group f = r / NA), in samples.
-template<class D> PB2_HD int halo_row(int r) { return (r >> D::RA) * D::GSTR + (r & (D::NA - 1)) * D::SPR; }
+template<class D> __device__ __forceinline__ int halo_row(int r) { return (r >> D::RA) * D::GSTR + (r & (D::NA - 1)) * D::SPR; }
 
 // Stage-2 input rows start at sample p of their delay lines, p mod 8 = ((r + 1) dm) mod 8 with the block's
 // dm; DM4 = dm mod 4 fixes the shift within a vector at compile time, and bit 2 of p is that of
@@ -297,7 +278,7 @@ template<class D> PB2_HD int halo_row(int r) { return (r >> D::RA) * D::GSTR + (
 //
 // Phase a of one tile of 'tile' samples at T by thread 'tid'; ring: the delay line at T.
 template<class D, int DM4>
-PB2_HD void halo_phase_a(int tid, int tile, int dm, const typename D::Ts *stg, float *ring, const int *tabw)
+__device__ __forceinline__ void halo_phase_a(int tid, int tile, int dm, const typename D::Ts *stg, float *ring, const int *tabw)
 {
     constexpr int NA = D::NA, NB = D::NB, RA = D::RA, O = halo_org(RA);
     const int warp = tid >> 5, lane = tid & 31;
@@ -363,7 +344,7 @@ PB2_HD void halo_phase_a(int tid, int tile, int dm, const typename D::Ts *stg, f
 
 // Phase b of one tile by thread 'tid': thread (d, tl); emit(f, x) takes output row f's 4 samples.
 template<class D, typename Emit>
-PB2_HD void halo_phase_b(int tid, int tile, const float *ring, const int *tabr, Emit emit)
+__device__ __forceinline__ void halo_phase_b(int tid, int tile, const float *ring, const int *tabr, Emit emit)
 {
     constexpr int NB = D::NB, RB = D::RB, O = halo_org(RB);
     const int d = tid / D::TL, tl = tid % D::TL;
@@ -386,8 +367,8 @@ PB2_HD void halo_phase_b(int tid, int tile, const float *ring, const int *tabr, 
     });
 #pragma unroll
     for (int f = 0; f < NB; f++) {
-        const float x[4] = {halo_out(v[f][O], D::SU), halo_out(v[f][O + 1], D::SU), halo_out(v[f][O + 2], D::SU),
-                            halo_out(v[f][O + 3], D::SU)};
+        const float x[4] = {tree_out(v[f][O], D::SU), tree_out(v[f][O + 1], D::SU), tree_out(v[f][O + 2], D::SU),
+                            tree_out(v[f][O + 3], D::SU)};
         emit(f, x);
     }
 }
@@ -397,7 +378,7 @@ PB2_HD void halo_phase_b(int tid, int tile, const float *ring, const int *tabr, 
 // of step r: even band pairs are the in-place butterflies, odd ("staggered") pairs (2k + 1, 2k + 2) extra ones.
 // cnt[l] bands and first multiplet mb[l] per level; emit(m, x) takes multiplet m's 4 samples.
 template<class D, typename Emit>
-PB2_HD void halo_phase_b_sub(int tid, int tile, const float *ring, const int *tabr, const int *cnt, const int *mb, Emit emit)
+__device__ __forceinline__ void halo_phase_b_sub(int tid, int tile, const float *ring, const int *tabr, const int *cnt, const int *mb, Emit emit)
 {
     constexpr int NB = D::NB, RB = D::RB, O = halo_org(RB), W = kHaloW;
     constexpr int SA = D::NORM ? 0 : D::RA;
@@ -425,7 +406,7 @@ PB2_HD void halo_phase_b_sub(int tid, int tile, const float *ring, const int *ta
 #pragma unroll
         for (int f = 0; f < NB; f++)
             if (f < cnt[0]) {
-                const float x[4] = {halo_out(v[f][O], SA), halo_out(v[f][O + 1], SA), halo_out(v[f][O + 2], SA), halo_out(v[f][O + 3], SA)};
+                const float x[4] = {tree_out(v[f][O], SA), tree_out(v[f][O + 1], SA), tree_out(v[f][O + 2], SA), tree_out(v[f][O + 3], SA)};
                 emit(mb[0] + f, x);
             }
     }
@@ -441,8 +422,8 @@ PB2_HD void halo_phase_b_sub(int tid, int tile, const float *ring, const int *ta
                     float x[4], y[4];
 #pragma unroll
                     for (int t = 0; t < W; t++) {
-                        x[t] = halo_out(halo_bfly<D::NORM>(v[qa][t - L + O], v[qb][t + O]), S);
-                        y[t] = halo_out(halo_bfly<D::NORM>(v[qa][t - L - 1 + O], v[qb][t + O]), S);
+                        x[t] = tree_out(bfly_n<D::NORM>(v[qa][t - L + O], v[qb][t + O]), S);
+                        y[t] = tree_out(bfly_n<D::NORM>(v[qa][t - L - 1 + O], v[qb][t + O]), S);
                     }
                     const int m = m0 + (2 * k + 1) * (2 << r) + 2 * bitrev_c(j, r);
                     emit(m, x);
@@ -468,8 +449,8 @@ PB2_HD void halo_phase_b_sub(int tid, int tile, const float *ring, const int *ta
                 const int i0 = ((q >> r) << (r + 1)) | (q & (h - 1)), k = q >> r, j = q & (h - 1);
                 if (2 * k < c) {
                     const int m = m0 + (2 * k) * (2 << r) + 2 * bitrev_c(j, r);
-                    const float x[4] = {halo_out(v[i0][O], S), halo_out(v[i0][O + 1], S), halo_out(v[i0][O + 2], S), halo_out(v[i0][O + 3], S)};
-                    const float y[4] = {halo_out(v[i0 + h][O], S), halo_out(v[i0 + h][O + 1], S), halo_out(v[i0 + h][O + 2], S), halo_out(v[i0 + h][O + 3], S)};
+                    const float x[4] = {tree_out(v[i0][O], S), tree_out(v[i0][O + 1], S), tree_out(v[i0][O + 2], S), tree_out(v[i0][O + 3], S)};
+                    const float y[4] = {tree_out(v[i0 + h][O], S), tree_out(v[i0 + h][O + 1], S), tree_out(v[i0 + h][O + 2], S), tree_out(v[i0 + h][O + 3], S)};
                     emit(m, x);
                     emit(m + 1, y);
                 }
