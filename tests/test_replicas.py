@@ -121,3 +121,14 @@ def test_reference_arm_non_zero_rank_does_no_work():
     import bench
     args = argparse.Namespace(dtype="float16")
     assert bench.run_reference(args, 1, 2) is None
+
+
+def test_reference_arm_is_unavailable_without_the_reference(monkeypatch, capsys):
+    """Without pirate's compiled sources the arm says so; the oracle's restatement does not stand in."""
+    import json
+    import bench
+    monkeypatch.setattr(bench, "cpu_kind", lambda: "port")
+    monkeypatch.setattr("sys.argv", ["bench.py", "--impl", "reference"])
+    bench.main()
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
