@@ -19,8 +19,8 @@
 // so 8 warps have to hide the loads' latency with the trees' own parallelism (about 200 registers per thread);
 // measured on stage 1, 23 thread instructions per row and sample, issue 43% active, shared pipe 64%. The form with a
 // lane per sample, shuffled lags and kept histories executed 60. Four rank-16 beams, fp16, five trees, 2048 samples:
-// stage 1 1.99 -> 1.27 ms, stage 2 2.39 -> 1.52 ms; sixteen rank-12 beams, three trees: 0.49 -> 0.26 and 0.61 ->
-// 0.32 ms. kHaloW = 4: the halo costs a third of a rank-4 tree's adds at 4 samples and half as much at 8, but 8 would
+// stage 1 1.99 -> 1.26 ms, stage 2 2.39 -> 1.49 ms; sixteen rank-12 beams, three trees: 0.49 -> 0.23 and 0.61 ->
+// 0.24 ms. kHaloW = 4: the halo costs a third of a rank-4 tree's adds at 4 samples and half as much at 8, but 8 would
 // leave a rank-8 block 4 warps.
 //
 // Alignment is known at compile time everywhere. Phase a's input rows start at sample p with
