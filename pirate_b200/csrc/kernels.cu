@@ -34,8 +34,9 @@ namespace pb2 {
 // 2^s1dd - 1 - (c mod 2^s1dd) (ReferenceLaggedDownsamplingKernel.cpp:46-57), so that the stage-1
 // kernel reads aligned rows.
 //
-// grid_lds_kernel, for chunk lengths or level counts that grid_warp_kernel below does not take: one thread per (beam,
-// tree-channel pair (2c, 2c+1), window of W0 level-0 samples); consecutive threads take consecutive windows, so every load and store is a contiguous run across the warp.
+// grid_lds_kernel, for the chunk lengths, level counts and int4 plans that grid_warp_kernel below does not take
+// (grid_warp_ok): one thread per (beam, tree-channel pair (2c, 2c+1), window of W0 level-0 samples); consecutive
+// threads take consecutive windows, so every load and store is a contiguous run across the warp.
 // The thread grids both channels of its window (and writes them as the level-0 tree), builds every
 // level in registers, and gets the even channel's predecessor sample at each level by gridding the
 // 2^nlev samples before its window (at the chunk start: from a parity double-buffered state).
